@@ -176,7 +176,7 @@ int make_expert_set(const imx_moe_config& c, const QFormat& f, const imx_qtensor
 bool is_prefill(int path) {
     return path == IMX_PATH_PREFILL || path == IMX_PATH_PREFILL_SMEM || path == IMX_PATH_PREFILL_PLAIN;
 }
-int unit_rows_for(int path) { return is_prefill(path) ? kPrefillUnitRows : kUnitRows; }
+int unit_rows_for(int path) { return is_prefill(path) || path == kPathTwoTerm ? kPrefillUnitRows : kUnitRows; }
 bool is_decode(int path) { return path == IMX_PATH_DECODE || path == IMX_PATH_DECODE_REGS; }
 bool decode_supported(const ExpertSet& s) { return decode_mma_supported(s) || decode_fp_supported(s); }
 
@@ -187,7 +187,8 @@ int pick_path(const imx_moe_config& c, const ExpertSet& s, long n_rows, int* pat
     const bool many = n_rows >= 32L * s.num_experts;
     if (p == IMX_PATH_AUTO) {
         if (many && prefill_tc_supported(s)) p = IMX_PATH_PREFILL;
-        else p = decode_supported(s) ? IMX_PATH_DECODE : IMX_PATH_GENERIC;
+        else if (decode_supported(s)) p = IMX_PATH_DECODE;
+        else p = two_term_supported(s) && two_term_aligned(s) ? kPathTwoTerm : IMX_PATH_GENERIC;
     }
     IMX_REQUIRE(!(p == IMX_PATH_PREFILL || p == IMX_PATH_PREFILL_SMEM || p == IMX_PATH_PREFILL_PLAIN) || prefill_tc_supported(s),
                 "the prefill path supports affine 2/4/8-bit, mxfp8 and nvfp4 with hidden %% 128 == 0, intermediate %% 64 == 0 "
@@ -209,6 +210,7 @@ int run_experts(int path, const GroupedArgs& ga, cudaStream_t stream, cudaEvent_
     if (path == IMX_PATH_PREFILL) return launch_prefill_tc(ga, stream, mid, 0);
     if (path == IMX_PATH_PREFILL_PLAIN) return launch_prefill_tc(ga, stream, mid, 1);
     if (path == IMX_PATH_PREFILL_SMEM) return launch_prefill_tc(ga, stream, mid, 2);
+    if (path == kPathTwoTerm) return launch_prefill_tc(ga, stream, mid, 3);
     if (is_decode(path) && decode_fp_supported(ga.set)) return launch_decode_fp(ga, stream, mid);
     if (path == IMX_PATH_DECODE && decode_tmap_supported(ga.set)) return launch_decode_tmap(ga, stream, mid);
     if (is_decode(path)) return launch_decode_mma(ga, stream, mid);

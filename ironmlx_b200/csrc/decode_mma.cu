@@ -222,7 +222,8 @@ void decode_block_order(int bits, int order[16]) {
 }
 
 void expert_block_order(const QFormat& f, int order[16]) {
-    decode_block_order(f.mode == IMX_MODE_AFFINE ? f.bits : 0, order);
+    if (f.mode == IMX_MODE_AFFINE && (f.bits == 3 || f.bits == 5 || f.bits == 6)) two_term_block_order(f.bits, order);
+    else decode_block_order(f.mode == IMX_MODE_AFFINE ? f.bits : 0, order);
 }
 
 bool decode_mma_supported(const ExpertSet& s) {

@@ -391,6 +391,7 @@ int forward_gathered(imx_ep_ctx& x, const imx_moe_weights* w, const void* xin, i
         cd.path = IMX_PATH_DECODE;
         if (pick_path(cd, set, (long)A / R, &path) != IMX_OK) path = IMX_PATH_GENERIC;
     }
+    if (path == kPathTwoTerm) path = IMX_PATH_GENERIC;   // (the workspace of this schedule is not laid out for it)
     const bool tc = is_prefill(path);                // tensor-core kernels: fp16 rows, routing weight applied in the combine
     const bool tmap_decode = path == IMX_PATH_DECODE && decode_tmap_supported(set);
 

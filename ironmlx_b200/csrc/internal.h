@@ -157,6 +157,12 @@ constexpr int kPrefillUnitRows = 256;
 // activations everywhere; 2: the dequantized tile through shared memory (1 and 2 are cross-checks).
 bool prefill_tc_supported(const ExpertSet& s, bool second_only = false);
 int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid = nullptr, int variant = 0);
+// The same kernels with the weight as a two-term fp16 sum, for the formats whose weights stay in 32 bits: affine
+// 3/5/6-bit and 4-bit in groups of 32.  kPathTwoTerm is what pick_path answers for them (never a caller's request).
+constexpr int kPathTwoTerm = 100;
+void two_term_block_order(int bits, int order[16]);   // 3, 5, 6 bits (4: the decode kernels' order)
+bool two_term_supported(const ExpertSet& s, bool second_only = false);
+bool two_term_aligned(const ExpertSet& s, bool second_only = false);
 // The current device: its ordinal and SM count (cached per device).
 struct DeviceInfo {
     int ordinal;

@@ -29,10 +29,30 @@ namespace {
 __global__ void __launch_bounds__(256)
 prepare_one_kernel(const __nv_bfloat16* __restrict__ src, int m, int cols, __half* __restrict__ dst, const Order16 order,
                    int unit_rows, int32_t* __restrict__ offsets, int32_t* __restrict__ ident, WorkUnit* __restrict__ units,
-                   int32_t* __restrict__ n_units, int32_t* __restrict__ sched, int sched_ints, float* __restrict__ psum) {
+                   int32_t* __restrict__ n_units, int32_t* __restrict__ sched, int sched_ints, float* __restrict__ psum,
+                   float* __restrict__ row_scale) {
     if ((int)blockIdx.x < m) {
         const size_t r = blockIdx.x;
         const __nv_bfloat16* s = src + r * cols;
+        if (row_scale != nullptr) {
+            // any bf16 row fits fp16 once its largest magnitude is brought into [2^14, 2^15) by a power of two, which
+            // the output gets back: row_scale = 2^-k.  Rows of zeros and rows with infinities or NaNs stay as they are.
+            __shared__ uint32_t s_mag[8];
+            uint32_t mag = 0;
+            for (int i = threadIdx.x; i < cols; i += blockDim.x) mag = max(mag, (uint32_t)__bfloat16_as_ushort(s[i]) & 0x7fffu);
+            mag = __reduce_max_sync(0xffffffffu, mag);
+            if ((threadIdx.x & 31) == 0) s_mag[threadIdx.x >> 5] = mag;
+            __syncthreads();
+            for (int w = 0; w < 8; ++w) mag = max(mag, s_mag[w]);
+            const int e = (int)(mag >> 7);
+            const int k = mag == 0 || e == 255 ? 0 : 141 - e;                 // -113 .. 141
+            const float up0 = __uint_as_float((uint32_t)(k / 2 + 127) << 23), up1 = __uint_as_float((uint32_t)(k - k / 2 + 127) << 23);
+            const float dn0 = __uint_as_float((uint32_t)(127 - k / 2) << 23), dn1 = __uint_as_float((uint32_t)(127 - (k - k / 2)) << 23);
+            for (int i = threadIdx.x; i < cols; i += blockDim.x)
+                dst[r * cols + i] = __float2half_rn(__bfloat162float(s[(i & ~15) + order.o[i & 15]]) * up0 * up1);
+            if (threadIdx.x == 0) row_scale[r] = dn0 * dn1;
+            return;
+        }
         for (int i = threadIdx.x; i < cols; i += blockDim.x) {
             const float v = __bfloat162float(s[(i & ~15) + order.o[i & 15]]);
             dst[r * cols + i] = __float2half_rn((i & 2) ? v * order.pair_scale_odd : v);
@@ -88,6 +108,7 @@ struct OneWs {
     float* psum;          // [m, K / 16 + 1]
     float* gsum_x;        // [m, in / 64 + 1]
     float* rows;          // [m, out] fp32 (or fp16 in the same buffer)
+    float* row_scale;     // [m] two-term path: what undoes the rows' power-of-two scaling
     int max_units;
     size_t bytes;
 };
@@ -110,6 +131,7 @@ OneWs carve_one(int m, int in, int mid, int out, void* base) {
     w.psum = cv.take<float>((size_t)m * (kmax / 16 + 1));
     w.gsum_x = cv.take<float>((size_t)m * (in / 64 + 1));
     w.rows = cv.take<float>((size_t)m * out);
+    w.row_scale = cv.take<float>((size_t)m);
     w.bytes = align_up(cv.off, 256);
     return w;
 }
@@ -149,6 +171,7 @@ int qmm_path(const ExpertSet& s, int m) {
     if (m >= 32 && prefill_tc_supported(s, true)) return IMX_PATH_PREFILL;
     if (m <= 256 && (decode_tmap_supported(s) || decode_mma_supported(s) || decode_fp_supported(s))) return IMX_PATH_DECODE;
     if (prefill_tc_supported(s, true)) return IMX_PATH_PREFILL;
+    if (two_term_supported(s, true)) return kPathTwoTerm;
     return IMX_PATH_GENERIC;
 }
 
@@ -275,7 +298,8 @@ int imx_quantized_matmul_ws(const void* x, int m, const imx_qtensor* w, int n_ou
     order.pair_scale_odd = tmap_second ? 0.0625f : 1.f;
     prepare_one_kernel<<<m + 1, 256, 0, stream>>>((const __nv_bfloat16*)x, m, in, ws.x16, order, unit_rows_for(path), ws.offsets,
                                                   ws.ident, ws.units, ws.n_units, ws.sw.sched, ws.sw.n_ints,
-                                                  tmap_second ? ws.psum : nullptr); IMX_LAUNCHED();
+                                                  tmap_second ? ws.psum : nullptr,
+                                                  path == kPathTwoTerm ? ws.row_scale : nullptr); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     GroupedArgs ga = {};
     ga.set = set;
@@ -290,6 +314,7 @@ int imx_quantized_matmul_ws(const void* x, int m, const imx_qtensor* w, int n_ou
     ga.act = ws.x16;                 // the second product reads its activations here
     ga.act_stride = in;
     ga.out = ws.rows;
+    ga.row_scale = path == kPathTwoTerm ? ws.row_scale : nullptr;
     ga.status = ws.status;
     IMX_TRY(run_experts(path, ga, stream));
     return launch_combine(ws.rows, nullptr, ws.ident, m, 1, n_out, nullptr, y, stream);
@@ -329,7 +354,7 @@ int imx_expert_forward(const imx_moe_config* cfg, const imx_qtensor* gate_up, co
     order.pair_scale_odd = tmap ? 0.0625f : 1.f;
     prepare_one_kernel<<<m + 1, 256, 0, stream>>>((const __nv_bfloat16*)x, m, c.hidden, ws.x16, order, unit_rows_for(path),
                                                   ws.offsets, ws.ident, ws.units, ws.n_units, ws.sw.sched, ws.sw.n_ints,
-                                                  nullptr); IMX_LAUNCHED();
+                                                  nullptr, nullptr); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     const bool rows_f16 = is_prefill(path);
     GroupedArgs ga = {};

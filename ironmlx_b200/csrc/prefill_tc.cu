@@ -66,9 +66,19 @@ constexpr uint32_t kTmemCols = 512;                // two 128-column accumulator
 constexpr uint32_t kTmemA = 256;                   // first column of the A ring (32 columns per stage)
 constexpr int kThreadsTc = 640;                    // 20 warps: 4 control, 4 + 4 epilogue, 8 producers
 
-enum { FMT_A4 = 0, FMT_A8 = 1, FMT_A2 = 2, FMT_MXFP8 = 3, FMT_NVFP4 = 4 };
-__host__ __device__ constexpr int q_row_bytes(int fmt) {       // packed bytes of one row per K step
-    return fmt == FMT_A8 || fmt == FMT_MXFP8 ? 64 : (fmt == FMT_A2 ? 16 : 32);
+// FMT_T*: affine weights as a two-term fp16 sum (hi + lo), see TwoTerm below.
+enum { FMT_A4 = 0, FMT_A8 = 1, FMT_A2 = 2, FMT_MXFP8 = 3, FMT_NVFP4 = 4, FMT_T3 = 5, FMT_T4 = 6, FMT_T5 = 7, FMT_T6 = 8 };
+__host__ __device__ constexpr bool two_term(int fmt) { return fmt >= FMT_T3; }
+__host__ __device__ constexpr int two_term_bits(int fmt) { return fmt - FMT_T3 + 3; }
+// Bytes of one row the copy engine brings per K step of 64 values.  3- and 5-bit rows advance by 24 and 40 bytes a
+// step and a copy starts on a multiple of 16: the box starts at the multiple below and is wide enough for both
+// positions.  48-byte rows spread eight lanes' 16-byte loads over all banks without a swizzle.
+__host__ __device__ constexpr int q_row_bytes(int fmt) {
+    return fmt == FMT_A8 || fmt == FMT_MXFP8 ? 64 : (fmt == FMT_A2 ? 16 : (fmt == FMT_T3 || fmt == FMT_T5 || fmt == FMT_T6 ? 48 : 32));
+}
+// First byte of K step ks's box in a packed row (a multiple of 16).
+__host__ __device__ constexpr int q_step_byte(int fmt, int ks) {
+    return fmt == FMT_T3 ? (ks * 24) & ~15 : (fmt == FMT_T5 ? (ks * 40) & ~15 : ks * q_row_bytes(fmt));
 }
 
 // Per-role cycle counters of CTA 0, compiled in only for timing experiments (-DIMX_TC_PROFILE).
@@ -221,6 +231,21 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
           "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// 16 consecutive columns of this thread's lane <- v; the caller waits with tmem_st_wait
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
 }
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
@@ -499,6 +524,86 @@ struct Dequant<FMT_NVFP4> {
     }
 };
 
+// ── two-term weights ────────────────────────────────────────────────────────
+// The formats no 16-bit kernel served before (affine 3/5/6-bit, and 4-bit in groups of 32) had their weights in fp32
+// in the scalar kernel.  One fp16 rounding of s * q + b would be a loss, so the MMA gets the weight as a sum of two
+// fp16 terms, hi + lo, good to 22 bits, with two MMAs per 16 values: the tile of A is 64 tensor-memory columns per
+// K step.  Everything is exact but the last rounding of lo:
+//   p = rn(q * s), e = q * s - p           exact: s is a bf16 value (8 bits), q has at most 6
+//   hi = rn(p + b), lo = rn(e + err)       err = the rounding error of p + b (two-sum)
+// fp16's range is met by a power of two 2^k per weight row, from the row's largest |s| 2^bits or |b|, taken back in
+// the epilogue (fp32).  Measured on a B200 against the scalar kernels, 1000 tokens over 256 experts of 2048 x 512, 6-bit:
+// both products 5.65 ms -> 0.52 ms (the block 5.74 -> 0.57 ms); what bounds it now is the MMAs' issue (eight per K step
+// whatever their N) beside the dequantization, two thirds of a K step's time.  Codes are pulled out in pairs (a, a + D) of a window of the bit stream, so that the second
+// one lands in the upper half-word HS bits up (that factor goes into its copy of the scale); codes of a block of 16
+// that have no partner at that distance pair with their neighbour.
+template <int BITS>
+struct TwoTerm {
+    static constexpr int D = BITS == 3 ? 6 : (BITS == 6 ? 3 : 4);
+    static constexpr int HS = BITS * D - 16;                 // bit of the upper half-word the second code starts at
+    static constexpr int SPAN = BITS == 3 ? 12 : (BITS == 6 ? 6 : 8);   // codes that pair up among themselves
+    // first code of pair p of a block of 16 and the distance of its partner
+    __host__ __device__ static constexpr int first(int p) {
+        const int full = 16 / SPAN * SPAN, rest = p - full / 2;
+        if (rest < 0) return p / D * SPAN + p % D;
+        if (BITS == 6) return rest == 0 ? 12 : 13;           // (12, 15) (13, 14)
+        return full + 2 * rest;
+    }
+    __host__ __device__ static constexpr int dist(int p) {
+        const int full = 16 / SPAN * SPAN, rest = p - full / 2;
+        if (rest < 0) return D;
+        return BITS == 6 && rest == 0 ? 3 : 1;
+    }
+    // the pair as 1024 + q (lower half), 1024 + 2^HS q (upper half)
+    template <int BIT, int DIST>
+    static __device__ __forceinline__ uint32_t pair(const uint32_t* w) {
+        constexpr uint32_t m = (1u << BITS) - 1u;
+        constexpr int i = BIT >> 5, sh = BIT & 31, need = DIST * BITS + BITS;
+        uint32_t v, r;
+        if constexpr (sh + need <= 32) v = w[i] >> sh;
+        else v = __funnelshift_r(w[i], w[i + 1], sh);
+        if constexpr (DIST == D) {
+            asm("lop3.b32 %0, %1, %2, 0x64006400, 0xea;" : "=r"(r) : "r"(v), "n"(m | (m << (16 + HS))));
+        } else {
+            const uint32_t u = v << (16 + HS - DIST * BITS);
+            asm("lop3.b32 %0, %1, %2, 0x64006400, 0xea;" : "=r"(r) : "r"(v), "n"(m));
+            asm("lop3.b32 %0, %1, %2, %0, 0xea;" : "+r"(r) : "r"(u), "n"(m << (16 + HS)));
+        }
+        return r;
+    }
+    // two blocks of 16 values of one group (block BLK of the 64 on): 16 registers of hi pairs, 16 of lo pairs
+    template <int BLK, int P>
+    static __device__ __forceinline__ void one(const uint32_t* w, __half2 s, __half2 b, uint32_t* hi_out, uint32_t* lo_out) {
+        const __half2 q = __hsub2(bits_h2(pair<BLK * 16 * BITS + first(P) * BITS, dist(P)>(w)), __float2half2_rn(1024.f));
+        const __half2 pr = __hmul2_rn(q, s);
+        const __half2 hi = __hadd2_rn(pr, b);
+        const __half2 bb = __hsub2_rn(hi, pr);
+        __half2 lo = __hadd2_rn(__hsub2_rn(pr, __hsub2_rn(hi, bb)), __hsub2_rn(b, bb));
+        if (BITS > 3) lo = __hadd2_rn(lo, __hfma2(q, s, __hneg2(pr)));   // 3 + 8 bits: the product is exact
+        *hi_out = h2_bits(hi);
+        *lo_out = h2_bits(lo);
+    }
+    template <int BLK>
+    static __device__ __forceinline__ void block(const uint32_t* w, __half2 s, __half2 b, uint32_t* hi, uint32_t* lo) {
+        one<BLK, 0>(w, s, b, hi + 0, lo + 0); one<BLK, 1>(w, s, b, hi + 1, lo + 1);
+        one<BLK, 2>(w, s, b, hi + 2, lo + 2); one<BLK, 3>(w, s, b, hi + 3, lo + 3);
+        one<BLK, 4>(w, s, b, hi + 4, lo + 4); one<BLK, 5>(w, s, b, hi + 5, lo + 5);
+        one<BLK, 6>(w, s, b, hi + 6, lo + 6); one<BLK, 7>(w, s, b, hi + 7, lo + 7);
+    }
+};
+__device__ __forceinline__ float pow2_f32(int e) {           // e in [-126, 127]
+    return __uint_as_float((uint32_t)(e + 127) << 23);
+}
+// Running maximum over eight scales (or biases) of a row as bf16 magnitudes, `up` added to the exponent of each.
+__device__ __forceinline__ uint32_t max_mag(uint4 v, uint32_t up, uint32_t m) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m = __vmaxu2(m, (w[i] & 0x7fff7fffu) + up);
+    return m;
+}
+// The exponent k of the row's power of two: its largest |s| 2^bits or |b| comes to lie in [2^13, 2^14).
+__device__ __forceinline__ int row_shift(uint32_t mag2) { return 140 - (int)(max(mag2 & 0xffffu, mag2 >> 16) >> 7); }
+
 // 2^d (d <= 0) as an fp16 bit pattern in both halves; below 2^-24 it is zero.
 __device__ __forceinline__ __half2 pow2_half2(int d) {
     uint32_t b = 0;
@@ -527,9 +632,13 @@ template <bool SWIGLU, int FMT, bool TS, bool WIDE, bool XR>
 __global__ void __launch_bounds__(kThreadsTc, 1)
 prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__ TcMaps maps) {
     static_assert(!WIDE || (TS && !XR), "wide tiles: tensor-memory operand, streamed activations");
+    constexpr bool TWO = two_term(FMT);
+    static_assert(!TWO || (TS && WIDE), "two-term weights: 256-slot tiles, tensor-memory operand");
+    constexpr int ACOLS = TWO ? 64 : 32;                     // tensor-memory columns of one stage's A tile
+    constexpr int TBITS = TWO ? two_term_bits(FMT) : 4;
     constexpr int QROW = q_row_bytes(FMT);
     constexpr int QBYTES = 128 * QROW;                       // packed codes of one 128-row tile per K step
-    constexpr bool AFFINE = FMT == FMT_A4 || FMT == FMT_A8 || FMT == FMT_A2;
+    constexpr bool AFFINE = FMT == FMT_A4 || FMT == FMT_A8 || FMT == FMT_A2 || TWO;
     constexpr int XB = WIDE ? 2 * kXBytes : kXBytes;         // activation tile of a stage
     constexpr uint32_t Q_OFF = XR ? 0u : (uint32_t)(XB + (TS ? 0 : kWBytes));
     constexpr int NB = WIDE ? 1 : 2;                         // accumulator buffers
@@ -597,8 +706,9 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
 #pragma unroll
                     for (int kk = 0; kk < kTileK / 16; ++kk) {
                         const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
-                        if (TS) umma_ts(d, tmem + kTmemA + (uint32_t)(r.s * 32 + kk * 8), dx + 2 * kk, idesc, acc);
+                        if (TS) umma_ts(d, tmem + kTmemA + (uint32_t)(r.s * ACOLS + kk * 8), dx + 2 * kk, idesc, acc);
                         else umma_ss(d, smem_desc(stage + XB) + 2 * kk, dx + 2 * kk, idesc, acc);
+                        if (TWO) umma_ts(d, tmem + kTmemA + (uint32_t)(r.s * ACOLS + 32 + kk * 8), dx + 2 * kk, idesc, 1u);
                     }
                     umma_commit(smem_u32(&bars->empty[r.s]));                // stage free once these MMAs retire
                     if (ks == ksteps - 1) umma_commit(smem_u32(&bars->acc_full[buf]));
@@ -654,8 +764,8 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                         tma_load_2d(xdst, &maps.x, ks * kTileK, t.slot0, bar);
                         if (two) tma_load_2d(xdst + kXBytes, &maps.x, ks * kTileK, t.slot0 + 128, bar);
                     }
-                    tma_load_2d(stage + Q_OFF, &maps.w[mi0], ks * QROW, row0, bar);
-                    tma_load_2d(stage + Q_OFF + QBYTES / 2, &maps.w[mi1], ks * QROW, row1, bar);
+                    tma_load_2d(stage + Q_OFF, &maps.w[mi0], q_step_byte(FMT, ks), row0, bar);
+                    tma_load_2d(stage + Q_OFF + QBYTES / 2, &maps.w[mi1], q_step_byte(FMT, ks), row1, bar);
                 }
                 __syncwarp();
                 r.advance(1, stages);
@@ -674,8 +784,19 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
             if (!WIDE && buf != eh) return true;                    // two accumulators: one set of four warps each
             const ExpertSet& S = a.set;
             // Per-row output factors (before the accumulator is waited for: global loads): nvfp4's tensor scale,
-            // mxfp8's 2^(largest scale exponent of the row - 127).
+            // mxfp8's 2^(largest scale exponent of the row - 127), two-term weights' 2^-k.
             auto row_factor = [&](const QMat& m, size_t estride, int r_in) -> float {
+                if (TWO) {
+                    const int srow = (t.K >> p.lg_group) * 2;
+                    const size_t off = (t.extra ? 0 : (size_t)t.expert * estride) + (size_t)r_in * srow;
+                    uint32_t mx = 0;
+                    for (int i = 0; i < srow; i += 16) {
+                        mx = max_mag(__ldg(reinterpret_cast<const uint4*>(m.scales + off + i)), (uint32_t)TBITS * 0x00800080u, mx);
+                        mx = max_mag(__ldg(reinterpret_cast<const uint4*>(m.biases + off + i)), 0u, mx);
+                    }
+                    const int k = row_shift(mx);
+                    return pow2_f32(-(k / 2)) * pow2_f32(-(k - k / 2));
+                }
                 if (AFFINE) return 1.f;
                 if (FMT == FMT_NVFP4) return m.global_scale;
                 const int srow = t.K >> 5;                          // one ue8m0 byte per 32 values
@@ -724,7 +845,7 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                         for (int j = 0; j < 8; ++j) {
                             float g0 = __uint_as_float(v[4 * j]), g1 = __uint_as_float(v[4 * j + 1]);
                             float u0 = __uint_as_float(v[4 * j + 2]), u1 = __uint_as_float(v[4 * j + 3]);
-                            if (!AFFINE) { g0 *= rf[2 * gs]; g1 *= rf[2 * gs]; u0 *= rf[2 * gs + 1]; u1 *= rf[2 * gs + 1]; }
+                            if (!AFFINE || TWO) { g0 *= rf[2 * gs]; g1 *= rf[2 * gs]; u0 *= rf[2 * gs + 1]; u1 *= rf[2 * gs + 1]; }
                             const float r0 = silu_fast(g0) * u0, r1 = silu_fast(g1) * u1;
                             peak = fmaxf(peak, fmaxf(fabsf(r0), fabsf(r1)));
                             o[j] = pack_f16_sat(r0, r1);
@@ -756,12 +877,14 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                     if (a.row_scale != nullptr) {
                         // a weight per slot: one per lane, handed round by shuffle
                         const int my = c * 32 + lane;
-                        const float rs = (my < t.rows ? a.row_scale[t.slot0 + my] : 1.f) * rf[0];
+                        // (the weight row's own factor, rf, belongs to the lane and is not handed round)
+                        const float rs = my < t.rows ? a.row_scale[t.slot0 + my] : 1.f;
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) o[i] = __uint_as_float(v[i]) * __shfl_sync(0xffffffffu, rs, i);
+                        for (int i = 0; i < 32; ++i)
+                            o[i] = (AFFINE && !TWO ? __uint_as_float(v[i]) : __uint_as_float(v[i]) * rf[0]) * __shfl_sync(0xffffffffu, rs, i);
                     } else {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) o[i] = AFFINE ? __uint_as_float(v[i]) : __uint_as_float(v[i]) * rf[0];
+                        for (int i = 0; i < 32; ++i) o[i] = AFFINE && !TWO ? __uint_as_float(v[i]) : __uint_as_float(v[i]) * rf[0];
                     }
                     const size_t o0 = (size_t)(t.slot0 + c * 32) * a.set.n_in + col;
                     const int n_ok = t.rows - c * 32;
@@ -828,6 +951,17 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                 for (uint32_t i = 0; i < srow; i += 16) mx = max_byte(lds128(s_addr + i), mx);
                 r_exp = (int)hmax_bytes(mx);
             }
+            float up0 = 1.f, up1 = 1.f;               // two-term weights: the row's 2^k, as two factors in fp32's range
+            if (TWO) {
+                uint32_t mx = 0;
+                for (uint32_t i = 0; i < srow; i += 16) {
+                    mx = max_mag(lds128(s_addr + i), (uint32_t)TBITS * 0x00800080u, mx);
+                    mx = max_mag(lds128(b_addr + i), 0u, mx);
+                }
+                const int k = row_shift(mx);
+                up0 = pow2_f32(k / 2);
+                up1 = pow2_f32(k - k / 2);
+            }
             int ks = grp_id;
             for (; ks < ksteps; ks += 2) {
                 PROF_BEGIN
@@ -836,7 +970,41 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                 PROF_BEGIN
                 const uint32_t stage = sbase + (uint32_t)(r.s * p.stage_bytes);
                 uint32_t out[32];
-                if (AFFINE) {
+                if constexpr (TWO) {
+                    using Tt = TwoTerm<TBITS>;
+                    // the step's 64 codes of this row as a bit stream
+                    uint32_t w[2 * TBITS];
+                    if (TBITS == 6 || TBITS == 4) {
+#pragma unroll
+                        for (int c = 0; c < TBITS / 2; ++c) {
+                            const uint4 v = lds128(stage + q_off + (((uint32_t)c ^ (TBITS == 4 ? swz : 0u)) << 4));
+                            w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
+                        }
+                    } else {
+                        const uint32_t at = stage + q_off + (uint32_t)(ks & 1) * 8u;   // 24 ks or 40 ks, less the box's start
+#pragma unroll
+                        for (int c = 0; c < TBITS; ++c) {
+                            const uint2 v = lds64(at + 8u * c);
+                            w[2 * c] = v.x; w[2 * c + 1] = v.y;
+                        }
+                    }
+                    const uint32_t ta = t_lane + (uint32_t)(r.s * ACOLS);
+                    auto half_step = [&](auto hc) {
+                        constexpr int h = decltype(hc)::value;
+                        const uint32_t gi = (uint32_t)(ks * kTileK + h * 32) >> p.lg_group;
+                        const float sf = __uint_as_float(lds16(s_addr + gi * 2) << 16) * up0 * up1;
+                        const float bf = __uint_as_float(lds16(b_addr + gi * 2) << 16) * up0 * up1;
+                        const __half2 s2 = __floats2half2_rn(sf, sf * (1.f / (float)(1 << Tt::HS)));
+                        const __half2 b2 = __float2half2_rn(bf);
+                        uint32_t hi[16], lo[16];
+                        Tt::template block<2 * h>(w, s2, b2, hi, lo);
+                        Tt::template block<2 * h + 1>(w, s2, b2, hi + 8, lo + 8);
+                        tmem_st16(ta + 16u * h, hi);
+                        tmem_st16(ta + 32u + 16u * h, lo);
+                    };
+                    half_step(std::integral_constant<int, 0>{});
+                    half_step(std::integral_constant<int, 1>{});
+                } else if constexpr (AFFINE) {
                     __half2 sc[2], bi[2];
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
@@ -847,14 +1015,17 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                     if (FMT == FMT_A4) Dequant<FMT_A4>::run(stage + q_off, swz, sc, bi, out);
                     if (FMT == FMT_A8) Dequant<FMT_A8>::run(stage + q_off, swz, sc, bi, out);
                     if (FMT == FMT_A2) Dequant<FMT_A2>::run(stage + q_off, swz, sc, bi, out);
-                } else if (FMT == FMT_MXFP8) {
+                } else if constexpr (FMT == FMT_MXFP8) {
                     const uint32_t s2 = lds16(s_addr + (uint32_t)ks * 2);
                     __half2 mult[2] = {pow2_half2((int)(s2 & 0xffu) - r_exp), pow2_half2((int)(s2 >> 8) - r_exp)};
                     Dequant<FMT_MXFP8>::run(stage + q_off, swz, mult, mult, out);
                 } else {
                     Dequant<FMT_NVFP4>::run(stage + q_off, swz, lds32(s_addr + (uint32_t)ks * 4), out);
                 }
-                if (TS) {
+                if constexpr (TWO) {
+                    tmem_st_wait();
+                    tc_fence_before();
+                } else if constexpr (TS) {
                     tmem_st32(t_lane + (uint32_t)(r.s * 32), out);
                     tc_fence_before();
                 } else {
@@ -903,6 +1074,11 @@ int fmt_index(const QFormat& f) {
     return -1;
 }
 
+// The two-term form of a format, or -1.
+int two_term_index(const QFormat& f) {
+    return f.mode == IMX_MODE_AFFINE && f.bits >= 3 && f.bits <= 6 ? FMT_T3 + f.bits - 3 : -1;
+}
+
 int log2_exact(int v) {
     int l = 0;
     while ((1 << l) < v) ++l;
@@ -934,9 +1110,16 @@ int make_q_maps(const QMat& m, size_t rows, int K, const QFormat& f, int fmt, CU
     return IMX_OK;
 }
 
+constexpr size_t kSmemMost = 227 * 1024;
+
 template <int FMT>
 int configure() {
-    constexpr int kSmem = 227 * 1024;
+    constexpr int kSmem = (int)kSmemMost;
+    if constexpr (two_term(FMT)) {
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        return IMX_OK;
+    } else {
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
@@ -945,6 +1128,7 @@ int configure() {
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     return IMX_OK;
+    }
 }
 
 struct Plan {
@@ -957,6 +1141,18 @@ struct Plan {
 template <int FMT>
 int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, const TcMaps& mgu, const TcMaps& mdn, int sms,
                cudaStream_t stream, cudaEvent_t mid) {
+    if constexpr (two_term(FMT)) {
+        if (!a.second_only) {
+            prefill_tc_kernel<true, FMT, true, true, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+            IMX_LAUNCHED();
+            IMX_CHECK_CUDA(cudaGetLastError());
+        }
+        if (mid) IMX_CHECK_CUDA(cudaEventRecord(mid, stream));
+        prefill_tc_kernel<false, FMT, true, true, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        IMX_LAUNCHED();
+        IMX_CHECK_CUDA(cudaGetLastError());
+        return IMX_OK;
+    } else {
     if (!a.second_only) {
         if (!ts) prefill_tc_kernel<true, FMT, false, false, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
         else if (gu.wide) prefill_tc_kernel<true, FMT, true, true, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
@@ -972,6 +1168,34 @@ int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, co
     IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     return IMX_OK;
+    }
+}
+
+// Shared memory of a launch: [panel][stages][two scale buffers][control block].  As many stages as fit,
+// at most 8 (4 with two-term weights: the ring of A tiles in tensor memory has 256 columns) and, with a resident
+// panel, at most the shortest reduction's K steps (the ring's back-pressure then also guards the panel).
+bool make_plan(const QFormat& f, int fmt, int K_max, int K_min, bool wide, bool xr, bool ts, Plan* out) {
+    const size_t q_tile = 128u * (size_t)q_row_bytes(fmt);
+    const size_t sc = (size_t)128 * scale_row(K_max, f) * (f.mode == IMX_MODE_AFFINE ? 2 : 1);
+    const size_t panel = xr ? (size_t)(K_max / kTileK) * kXBytes : 0;
+    const size_t stage = (xr ? 0 : (size_t)kXBytes * (wide ? 2 : 1) + (ts ? 0 : kWBytes)) + q_tile;
+    const size_t fixed = panel + 2 * sc + sizeof(Bars) + 1024;
+    if (fixed + 2 * stage > kSmemMost) return false;
+    int st = (int)((kSmemMost - fixed) / stage);
+    const int most = two_term(fmt) ? 4 : kMaxStages;
+    if (st > most) st = most;
+    if (xr && st > K_min / kTileK) st = K_min / kTileK;
+    if (st < 2) return false;
+    out->p = TcParams{};
+    out->p.stages = st;
+    out->p.stage_bytes = (int)stage;
+    out->p.sc_bytes = (int)sc;
+    out->p.panel_bytes = (int)panel;
+    out->p.lg_group = log2_exact(f.group);
+    out->smem = fixed + (size_t)st * stage;
+    out->wide = wide;
+    out->xr = xr;
+    return true;
 }
 
 }  // namespace
@@ -994,17 +1218,53 @@ bool prefill_tc_supported(const ExpertSet& s, bool second_only) {
     return true;
 }
 
-// variant: 0 = the shipped configuration (tensor-memory operand, 256-slot tiles in both products), 1 =
+template <int BITS>
+static void two_term_order(int order[16]) {
+    for (int p = 0; p < 8; ++p) {
+        order[2 * p] = TwoTerm<BITS>::first(p);
+        order[2 * p + 1] = TwoTerm<BITS>::first(p) + TwoTerm<BITS>::dist(p);
+    }
+}
+void two_term_block_order(int bits, int order[16]) {
+    if (bits == 3) two_term_order<3>(order);
+    else if (bits == 5) two_term_order<5>(order);
+    else if (bits == 6) two_term_order<6>(order);
+    else two_term_order<4>(order);
+}
+
+bool two_term_supported(const ExpertSet& s, bool second_only) {
+    const QFormat& f = s.fmt;
+    const int fmt = two_term_index(f);
+    if (fmt < 0 || (f.bits == 4 && f.group != 32)) return false;
+    if (s.n_in % 128) return false;
+    // packed rows advance in whole 16-byte pieces (the pitch a tiled copy needs)
+    auto ok = [&](int K) { return k_ok(K, f) && packed_row_bytes(K, f.bits) % 16 == 0; };
+    if ((!second_only && !ok(s.n_in)) || !ok(s.n_mid) || (s.has_extra && !ok(s.x_mid))) return false;
+    const int mid_max = s.has_extra && s.x_mid > s.n_mid ? s.x_mid : s.n_mid;
+    Plan p;
+    return (second_only || make_plan(f, fmt, s.n_in, s.n_in, true, false, true, &p)) &&
+           make_plan(f, fmt, mid_max, mid_max, true, false, true, &p);
+}
+
+// What the copy engine asks of the matrices' addresses (the scalar kernel takes any 16 / 4-byte aligned tensor).
+bool two_term_aligned(const ExpertSet& s, bool second_only) {
+    auto ok = [](const QMat& m) { return (((uintptr_t)m.w | (uintptr_t)m.scales | (uintptr_t)m.biases) % 16) == 0; };
+    if (!ok(s.down) || (!second_only && !(ok(s.gate) && ok(s.up)))) return false;
+    return !s.has_extra || (ok(s.x_down) && (second_only || (ok(s.x_gate) && ok(s.x_up))));
+}
+
+// variant: 3 = two-term weights (the only one for the formats two_term_supported() names); 0 = the shipped configuration (tensor-memory operand, 256-slot tiles in both products), 1 =
 // tensor-memory operand, 128-slot tiles and streamed activations everywhere, 2 = as 1 with the dequantized
 // tile in shared memory (1, 2: cross-checks).
 int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid, int variant) {
-    IMX_REQUIRE(prefill_tc_supported(a.set, a.second_only != 0), "prefill path: format/shape not supported");
+    IMX_REQUIRE(variant == 3 ? two_term_supported(a.set, a.second_only != 0) : prefill_tc_supported(a.set, a.second_only != 0),
+                "prefill path: format/shape not supported");
     IMX_REQUIRE((a.row_index == nullptr || a.xs != nullptr || a.second_only) && a.n_slots > 0,
                 "prefill path: slot-ordered activation buffer missing");
     if (a.max_units == 0) return IMX_OK;
     const ExpertSet& s = a.set;
     const QFormat& f = s.fmt;
-    const int fmt = fmt_index(f);
+    const int fmt = variant == 3 ? two_term_index(f) : fmt_index(f);
     const bool ts = variant != 2;
     const int x_mid = s.has_extra ? s.x_mid : s.n_mid;
     const int mid_max = s.n_mid > x_mid ? s.n_mid : x_mid;
@@ -1018,42 +1278,28 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
         IMX_TRY(configure<FMT_A2>());
         IMX_TRY(configure<FMT_MXFP8>());
         IMX_TRY(configure<FMT_NVFP4>());
+        IMX_TRY(configure<FMT_T3>());
+        IMX_TRY(configure<FMT_T4>());
+        IMX_TRY(configure<FMT_T5>());
+        IMX_TRY(configure<FMT_T6>());
         device_mark_setup(di.ordinal, kSetupPrefillTc);
     }
 
-    // Shared memory of a launch: [panel][stages][two scale buffers][control block].  As many stages as fit,
-    // at most 8 (the ring of A tiles in tensor memory has 256 columns) and, with a resident panel, at most
-    // the shortest reduction's K steps (the ring's back-pressure then also guards the panel).
-    const size_t q_tile = 128u * (size_t)q_row_bytes(fmt);
     auto plan = [&](int K_max, int K_min, bool wide, bool xr, Plan* out) -> bool {
-        const size_t sc = (size_t)128 * scale_row(K_max, f) * (f.mode == IMX_MODE_AFFINE ? 2 : 1);
-        const size_t panel = xr ? (size_t)(K_max / kTileK) * kXBytes : 0;
-        const size_t stage = (xr ? 0 : (size_t)kXBytes * (wide ? 2 : 1) + (ts ? 0 : kWBytes)) + q_tile;
-        const size_t fixed = panel + 2 * sc + sizeof(Bars) + 1024;
-        const size_t room = 227 * 1024;
-        if (fixed + 2 * stage > room) return false;
-        int st = (int)((room - fixed) / stage);
-        if (st > kMaxStages) st = kMaxStages;
-        if (xr && st > K_min / kTileK) st = K_min / kTileK;
-        if (st < 2) return false;
-        out->p = TcParams{};
-        out->p.stages = st;
-        out->p.stage_bytes = (int)stage;
-        out->p.sc_bytes = (int)sc;
-        out->p.panel_bytes = (int)panel;
-        out->p.lg_group = log2_exact(f.group);
-        out->smem = fixed + (size_t)st * stage;
-        out->wide = wide;
-        out->xr = xr;
-        return true;
+        return make_plan(f, fmt, K_max, K_min, wide, xr, ts, out);
     };
     Plan gu = {}, dn = {};
+    if (variant == 3) {
+        IMX_REQUIRE((a.second_only || plan(s.n_in, s.n_in, true, false, &gu)) && plan(mid_max, mid_min, true, false, &dn),
+                    "two-term path: sizes exceed shared memory");
+    } else {
     if (!a.second_only && !(variant == 0 && plan(s.n_in, s.n_in, true, false, &gu)))
         IMX_REQUIRE(plan(s.n_in, s.n_in, false, false, &gu), "prefill path: sizes exceed shared memory");
     // second product: 256-slot tiles with streamed activations as well (c3: 276 us against 377 us with 128-slot
     // tiles and the activation panel resident); the resident panel where the wide stages do not fit
     if (!(variant == 0 && (plan(mid_max, mid_min, true, false, &dn) || plan(mid_max, mid_min, false, true, &dn))))
         IMX_REQUIRE(plan(mid_max, mid_min, false, false, &dn), "prefill path: sizes exceed shared memory");
+    }
     gu.p.nt_r = s.n_mid / 64;
     gu.p.nt_x = x_mid / 64;
     dn.p.nt_r = dn.p.nt_x = s.n_in / 128;
@@ -1099,6 +1345,10 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
         case FMT_A2: return launch_fmt<FMT_A2>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
         case FMT_MXFP8: return launch_fmt<FMT_MXFP8>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
         case FMT_NVFP4: return launch_fmt<FMT_NVFP4>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
+        case FMT_T3: return launch_fmt<FMT_T3>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
+        case FMT_T4: return launch_fmt<FMT_T4>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
+        case FMT_T5: return launch_fmt<FMT_T5>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
+        case FMT_T6: return launch_fmt<FMT_T6>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
     }
     set_error("prefill path: unknown format");
     return IMX_ERR_INVALID;

@@ -1,0 +1,85 @@
+"""The tensor-core kernels with two-term weights (affine 3/5/6-bit, 4-bit in groups of 32): the formats whose
+weights stay in 32 bits, against fp64 and against the scalar kernels they replace."""
+import numpy as np
+import pytest
+import torch
+
+from ironmlx_b200 import nn, ops
+from ironmlx_b200.workloads import MoEConfig
+from oracle import moe as O
+from gpu_util import bf16_to_np, moe_to_device, t_bf16
+from util import make_params
+
+pytestmark = pytest.mark.gpu
+
+FORMATS = [(3, 64), (5, 64), (6, 64), (4, 32), (6, 32), (3, 128)]
+
+
+def _layer(cuda, n_out, n_in, bits, group, seed, scale=0.02):
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(seed)
+    w = torch.randn(n_out, n_in, generator=gen, device=cuda) * scale
+    q = ops.quantize(w, group, bits)
+    wd = ops.dequantize(*q, group, bits, dtype=torch.float32).double()
+    return nn.QuantizedLinear(*q, group, bits), wd, gen
+
+
+def _check(y, x, wd, in_dim):
+    """One rounding to bf16 (half a unit in the last of 8 bits: 2^-8 of the value at most), 2^-22 per weight (two fp16
+    terms) and the fp32 sums: at most n + 2 roundings of 2^-24 each of the sum of magnitudes."""
+    xd = x.double()
+    ref = xd @ wd.T
+    mags = xd.abs() @ wd.abs().T
+    bound = 2.0 ** -8 * ref.abs() + (2.0 ** -22 + (in_dim + 2) * 2.0 ** -24) * mags
+    assert torch.isfinite(y).all()
+    assert ((y.double() - ref).abs() <= bound).all(), ((y.double() - ref).abs() / bound).max().item()
+
+
+@pytest.mark.parametrize("bits,group", FORMATS)
+@pytest.mark.parametrize("m,in_dim,out_dim", [(1, 2048, 512), (17, 1024, 128), (129, 512, 384), (257, 1024, 256)])
+def test_linear(cuda, bits, group, m, in_dim, out_dim):
+    layer, wd, gen = _layer(cuda, out_dim, in_dim, bits, group, 3)
+    if in_dim // group * 2 % 16 or in_dim * bits // 8 % 16:
+        pytest.skip("rows the copy engine does not take")
+    x = torch.randn(m, in_dim, generator=gen, device=cuda)
+    # differences of two weights of a group: what a weight rounded to 16 bits gets wrong
+    if m > 8:
+        x[1::2] = 0
+        i = torch.randint(0, in_dim // group, (x[1::2].shape[0],), generator=gen, device=cuda) * group
+        r = torch.arange(x[1::2].shape[0], device=cuda) * 2 + 1
+        x[r, i + torch.randint(0, group // 2, i.shape, generator=gen, device=cuda)] = 1.0
+        x[r, i + group // 2 + torch.randint(0, group // 2, i.shape, generator=gen, device=cuda)] = -1.0
+    x = x.to(torch.bfloat16)
+    _check(layer.forward_with_stream(x), x, wd, in_dim)
+
+
+@pytest.mark.parametrize("bits,group", [(6, 64), (3, 64)])
+@pytest.mark.parametrize("x_scale,w_scale", [(1e20, 1e-12), (1e-25, 1e10), (1e-3, 1e-6), (70000.0, 3.0)])
+def test_linear_outside_the_range_of_fp16(cuda, bits, group, x_scale, w_scale):
+    layer, wd, gen = _layer(cuda, 256, 512, bits, group, 5, w_scale)
+    x = (torch.randn(40, 512, generator=gen, device=cuda) * x_scale)
+    x[3] = 0
+    x[4] *= 1e-6
+    x = x.to(torch.bfloat16)
+    _check(layer.forward_with_stream(x), x, wd, 512)
+
+
+@pytest.mark.parametrize("bits,group", FORMATS)
+@pytest.mark.parametrize("tokens,experts,top_k,shared", [(1, 8, 2, 512), (70, 4, 2, 0), (300, 3, 2, 512)])
+def test_block(cuda, bits, group, tokens, experts, top_k, shared):
+    cfg = MoEConfig("two-term", tokens=tokens, hidden=1024, num_experts=experts, top_k=top_k, intermediate=512,
+                    shared_intermediate=shared, bits=bits, group_size=group, seed=9)
+    if 512 // group * 2 % 16:
+        pytest.skip("rows of scales the copy engine does not take")
+    x, p = make_params(cfg)
+    moe = moe_to_device(p, cuda)
+    xd = t_bf16(x, cuda)
+    a = bf16_to_np(moe.forward_with_stream(xd))
+    moe.check_status()
+    b = bf16_to_np(moe.forward_with_stream(xd, path="generic"))
+    ref = O.moe_forward(x, p).y
+    assert O.rel_l2(a, ref) <= 2e-3
+    # no further from the checker than the scalar kernels (2 %: values that fall on either side of a rounding)
+    assert O.rel_l2(a, ref) <= 1.02 * O.rel_l2(b, ref)
+    # both round the SwiGLU rows to fp16 and the result to bf16: single values differ by a step of each at most
+    assert np.abs(a - b).max() <= 2.0 ** -8 * np.abs(b).max() * 1.5
