@@ -37,7 +37,7 @@
 //                 64 fp16 values (exact codes, one HFMA2 / HMUL2 with the
 //                 group's scale) -> one tcgen05.st of 32 columns
 // Every wait is bounded; on expiry the CTA records a status, every role leaves
-// its loop and tensor memory is freed.  No thread-block clusters, no multicast.
+// its loop and tensor memory is freed.  Wide tiles run in clusters of two CTAs (PAIR below); no multicast loads.
 //
 // Scales: affine rounds s*q+b once to fp16.  nvfp4: q * (e4m3 block scale) is
 // exact in fp16, the fp32 tensor scale is applied in the epilogue.  mxfp8: the
@@ -144,6 +144,31 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// Arrival on the barrier at the same offset in CTA 0 of the cluster.  What it announces is in tensor memory (ordered by
+// the tcgen05 fences around it), so that it needs no fence of ordinary memory: with .release.cluster the producers and
+// the epilogue waited for their stores each time, and the first product took 553 instead of 410 us (c3).
+__device__ __forceinline__ void mbar_arrive_cta0(uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\t"
+        "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
+        "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar)
+        : "memory");
+}
+// One lane of the (converged) warp.  Issued under `lane == 0` a tcgen05.mma cost 94 cycles whatever its N, its operands
+// being moved to uniform registers one lane at a time; under elect.sync 51 (N = 16) to 74 (N = 128), 33 to 64 for a pair.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // Bounded wait; false (and the abort flag set) when it gives up or someone else did.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     for (int spin = 0; spin < kSpin; ++spin) {
@@ -169,9 +194,9 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
     return (uint64_t)((addr >> 4) & 0x3fffu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
-// kind::f16 instruction descriptor: D fp32, A/B fp16 K-major, M = 128, N = n
-__device__ __forceinline__ uint32_t idesc_for(int n) {
-    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+// kind::f16 instruction descriptor: D fp32, A/B fp16 K-major, M = m, N = n
+__device__ __forceinline__ uint32_t idesc_for(int m, int n) {
+    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 // D[tmem_d] (+)= A[tmem_a] * B[smem]: A from tensor memory
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
@@ -181,6 +206,22 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
+}
+// The same for a pair of CTAs (issued by CTA 0): M = 256, each CTA's 128 lanes of A and D in its own tensor memory,
+// each CTA's half of B's rows at the same offset of its own shared memory.
+__device__ __forceinline__ void umma_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// Arrival on the barrier at this offset in both CTAs once the MMAs issued so far have retired.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((uint16_t)3)
+                 : "memory");
 }
 __device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -309,14 +350,21 @@ struct TileInfo {
 // (unit part, weight tile), items dealt round-robin.  XR = true: a work item is a unit part with all its
 // weight tiles in turn (its activation panel stays in shared memory).  nt_r / nt_x: weight tiles per unit of
 // the routed experts / the extra expert.  body(tile, index) returns false to stop.
-template <bool SWIGLU, bool XR, bool SPLIT, typename F>
+// PAIR: the two CTAs of a cluster take neighbouring weight tiles of the same unit (nt_r and nt_x are even).
+template <bool SWIGLU, bool XR, bool SPLIT, bool PAIR, typename F>
 __device__ __forceinline__ void for_each_tile(const GroupedArgs& a, int nt_r, int nt_x, F&& body) {
+    const int rank = PAIR ? (int)(blockIdx.x & 1) : 0;
+    if (PAIR) {
+        nt_r >>= 1;
+        nt_x >>= 1;
+    }
+    const int first = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     const int n_r = a.n_units[1], n_x = a.n_units[0] - n_r;
     const int tiles_r = n_r * nt_r;
     const int parts = SPLIT ? 2 : 1;
     const int total = (XR ? n_r + n_x : tiles_r + n_x * nt_x) * parts;
     int it = 0;
-    for (int w0 = blockIdx.x; w0 < total; w0 += gridDim.x) {
+    for (int w0 = first; w0 < total; w0 += step) {
         const int part = SPLIT ? (w0 & 1) : 0;
         const int w = SPLIT ? (w0 >> 1) : w0;
         int unit, nt0, ntn = 1;
@@ -350,7 +398,7 @@ __device__ __forceinline__ void for_each_tile(const GroupedArgs& a, int nt_r, in
         t.extra = u.expert >= a.set.num_experts;
         t.K = SWIGLU ? a.set.n_in : (t.extra ? a.set.x_mid : a.set.n_mid);
         for (int nt = nt0; nt < nt0 + ntn; ++nt, ++it) {
-            t.ntile = nt;
+            t.ntile = PAIR ? 2 * nt + rank : nt;
             t.first = nt == nt0;
             if (!body(t, it)) return;
         }
@@ -628,9 +676,17 @@ __device__ __forceinline__ uint32_t hmax_bytes(uint32_t m) {
 // its N, is then covered by the 128 cycles it runs) with one accumulator of 256 columns and eight epilogue
 // warps; otherwise tiles of up to 128 slots and two accumulators, the epilogue of tile i overlapping the MMAs
 // of tile i+1.  XR: the unit part's activation panel stays in shared memory for all its weight tiles.
-template <bool SWIGLU, int FMT, bool TS, bool WIDE, bool XR>
-__global__ void __launch_bounds__(kThreadsTc, 1)
-prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__ TcMaps maps) {
+// PAIR (wide tiles): two CTAs of a cluster share the activation tile.  Their weight tiles are neighbours, M = 256 in
+// one `cta_group::2` MMA that CTA 0 issues; each CTA brings and keeps half of the tile's slots (16 instead of 32 KB
+// a K step, so that eight stages fit instead of five) and dequantizes its own 128 weight rows.  CTA 0's full and
+// acc_empty barriers collect both CTAs' arrivals, commits reach the empty and acc_full barriers of both.  Two CTAs on
+// their own each read the whole activation tile from L2 and waited for it with five stages in flight; measured on a
+// B200, both products: 8192 tokens over 256 experts of 2048 x 512, 4-bit 736 -> 580 us, 4096 tokens nvfp4 445 -> 356 us,
+// 1777 tokens 8-bit 417 -> 328 us, 16384 skewed tokens 2-bit 1303 -> 1032 us.  What bounds them now is the MMAs (M = 256,
+// N = 256: 128 cycles each, 512 of the 577 a K step takes in the first product) and the epilogue between tiles.
+template <bool SWIGLU, int FMT, bool TS, bool WIDE, bool XR, bool PAIR>
+__device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcParams& p, const TcMaps& maps) {
+    static_assert(!PAIR || WIDE, "pairs of CTAs: wide tiles");
     static_assert(!WIDE || (TS && !XR), "wide tiles: tensor-memory operand, streamed activations");
     constexpr bool TWO = two_term(FMT);
     static_assert(!TWO || (TS && WIDE), "two-term weights: 256-slot tiles, tensor-memory operand");
@@ -639,7 +695,7 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
     constexpr int QROW = q_row_bytes(FMT);
     constexpr int QBYTES = 128 * QROW;                       // packed codes of one 128-row tile per K step
     constexpr bool AFFINE = FMT == FMT_A4 || FMT == FMT_A8 || FMT == FMT_A2 || TWO;
-    constexpr int XB = WIDE ? 2 * kXBytes : kXBytes;         // activation tile of a stage
+    constexpr int XB = WIDE && !PAIR ? 2 * kXBytes : kXBytes;   // activation tile of a stage
     constexpr uint32_t Q_OFF = XR ? 0u : (uint32_t)(XB + (TS ? 0 : kWBytes));
     constexpr int NB = WIDE ? 1 : 2;                         // accumulator buffers
     constexpr int DCOLS = WIDE ? 256 : 128;                  // columns of one accumulator
@@ -658,12 +714,12 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
     if (tid == 0) {
         for (int s = 0; s < kMaxStages; ++s) {
             mbar_init(smem_u32(&bars->qfull[s]), 1);
-            mbar_init(smem_u32(&bars->full[s]), 4);
+            mbar_init(smem_u32(&bars->full[s]), PAIR ? 8 : 4);
             mbar_init(smem_u32(&bars->empty[s]), 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&bars->acc_full[b]), 1);
-            mbar_init(smem_u32(&bars->acc_empty[b]), WIDE ? 8 : 4);
+            mbar_init(smem_u32(&bars->acc_empty[b]), PAIR ? 16 : (WIDE ? 8 : 4));
             mbar_init(smem_u32(&bars->sfull[b]), 1);
             mbar_init(smem_u32(&bars->sempty[b]), 8);
         }
@@ -671,28 +727,39 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
-                     "r"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
+                         "r"(kTmemCols)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
+                         "r"(kTmemCols)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();                                // the peer's barriers are initialised before anyone arrives on them
     tc_fence_after();
+    const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
     const uint32_t tmem = bars->tmem_base;
 
-    if (warp == 0) {
+    if (warp == 0 && rank != 0) {
+        // CTA 0 issues the pair's MMAs
+    } else if (warp == 0) {
         // ── MMA issuer ──────────────────────────────────────────────────────
         Ring r = {0, 0u};
         PROF_DECL
-        for_each_tile<SWIGLU, XR, SPLIT>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
+        for_each_tile<SWIGLU, XR, SPLIT, PAIR>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
             const int buf = it % NB, round = it / NB;
             PROF_BEGIN
             if (!mbar_wait(smem_u32(&bars->acc_empty[buf]), (uint32_t)(round & 1) ^ 1u, abort_flag)) return false;
             PROF_END(0)
             tc_fence_after();
             const int ksteps = t.K / kTileK;
-            const uint32_t idesc = idesc_for((t.rows + 15) & ~15);
+            const uint32_t idesc = PAIR ? idesc_for(256, (t.rows + 31) & ~31) : idesc_for(128, (t.rows + 15) & ~15);
             const uint32_t d = tmem + (uint32_t)(buf * DCOLS);
             for (int ks = 0; ks < ksteps; ++ks) {
                 PROF_BEGIN
@@ -700,18 +767,26 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                 PROF_END(1)
                 tc_fence_after();
                 PROF_BEGIN
-                if (lane == 0) {
+                if (elect_one()) {
                     const uint32_t stage = sbase + (uint32_t)(r.s * p.stage_bytes);
                     const uint64_t dx = smem_desc(XR ? panel + (uint32_t)(ks * kXBytes) : stage);
 #pragma unroll
                     for (int kk = 0; kk < kTileK / 16; ++kk) {
                         const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
-                        if (TS) umma_ts(d, tmem + kTmemA + (uint32_t)(r.s * ACOLS + kk * 8), dx + 2 * kk, idesc, acc);
+                        const uint32_t ta = tmem + kTmemA + (uint32_t)(r.s * ACOLS + kk * 8);
+                        if (PAIR) umma_ts_pair(d, ta, dx + 2 * kk, idesc, acc);
+                        else if (TS) umma_ts(d, ta, dx + 2 * kk, idesc, acc);
                         else umma_ss(d, smem_desc(stage + XB) + 2 * kk, dx + 2 * kk, idesc, acc);
-                        if (TWO) umma_ts(d, tmem + kTmemA + (uint32_t)(r.s * ACOLS + 32 + kk * 8), dx + 2 * kk, idesc, 1u);
+                        if (TWO && PAIR) umma_ts_pair(d, ta + 32, dx + 2 * kk, idesc, 1u);
+                        else if (TWO) umma_ts(d, ta + 32, dx + 2 * kk, idesc, 1u);
                     }
-                    umma_commit(smem_u32(&bars->empty[r.s]));                // stage free once these MMAs retire
-                    if (ks == ksteps - 1) umma_commit(smem_u32(&bars->acc_full[buf]));
+                    if (PAIR) {
+                        umma_commit_pair(smem_u32(&bars->empty[r.s]));
+                        if (ks == ksteps - 1) umma_commit_pair(smem_u32(&bars->acc_full[buf]));
+                    } else {
+                        umma_commit(smem_u32(&bars->empty[r.s]));            // stage free once these MMAs retire
+                        if (ks == ksteps - 1) umma_commit(smem_u32(&bars->acc_full[buf]));
+                    }
                 }
                 __syncwarp();
                 PROF_END(2)
@@ -724,7 +799,7 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
         // ── loader (TMA): activation tile, packed codes, scales ─────────────
         Ring r = {0, 0u};
         PROF_DECL
-        for_each_tile<SWIGLU, XR, SPLIT>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
+        for_each_tile<SWIGLU, XR, SPLIT, PAIR>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
             const int ksteps = t.K / kTileK;
             int mi0, mi1, row0, row1;
             tile_rows<SWIGLU>(a, t, t.ntile, mi0, mi1, row0, row1);
@@ -746,8 +821,10 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                 }
             }
             __syncwarp();
-            // activation rows this tile needs: one box of 128 slots, a second one past 128 rows
-            const bool two = WIDE && t.rows > 128;
+            // activation rows this tile needs: one box of 128 slots, a second one past 128 rows; of a pair, each
+            // CTA brings its half of the slots
+            const bool two = WIDE && !PAIR && t.rows > 128;
+            const int xslot = t.slot0 + (PAIR ? (int)rank * (((t.rows + 31) & ~31) >> 1) : 0);
             for (int ks = 0; ks < ksteps; ++ks) {
                 PROF_BEGIN
                 if (!mbar_wait(smem_u32(&bars->empty[r.s]), r.ph ^ 1u, abort_flag)) return false;
@@ -761,7 +838,7 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                     mbar_expect_tx(bar, (uint32_t)(QBYTES + (with_x ? (two ? 2 * kXBytes : kXBytes) : 0)));
                     if (with_x) {
                         const uint32_t xdst = XR ? panel + (uint32_t)(ks * kXBytes) : stage;
-                        tma_load_2d(xdst, &maps.x, ks * kTileK, t.slot0, bar);
+                        tma_load_2d(xdst, &maps.x, ks * kTileK, xslot, bar);
                         if (two) tma_load_2d(xdst + kXBytes, &maps.x, ks * kTileK, t.slot0 + 128, bar);
                     }
                     tma_load_2d(stage + Q_OFF, &maps.w[mi0], q_step_byte(FMT, ks), row0, bar);
@@ -779,7 +856,7 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
         const int eh = warp >= 16 ? 1 : 0;                      // WIDE: which half of the tile's slots; else: which accumulator
         const int lane128 = q * 32 + lane;
         PROF_DECL
-        for_each_tile<SWIGLU, XR, SPLIT>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
+        for_each_tile<SWIGLU, XR, SPLIT, PAIR>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
             const int buf = it % NB, round = it / NB;
             if (!WIDE && buf != eh) return true;                    // two accumulators: one set of four warps each
             const ExpertSet& S = a.set;
@@ -826,7 +903,10 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
             auto release = [&]() {                                  // all of this warp's TMEM reads are done
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty[buf]));
+                if (lane == 0) {
+                    if (PAIR) mbar_arrive_cta0(smem_u32(&bars->acc_empty[buf]));
+                    else mbar_arrive(smem_u32(&bars->acc_empty[buf]));
+                }
             };
             if (SWIGLU) {
                 // pieces of 64 slots x 16 lanes: 8 gate rows and the 8 matching up rows; a thread finishes row
@@ -834,39 +914,94 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                 const int n64 = (t.rows + 63) >> 6;
                 const int c_lo = WIDE ? eh * 2 : 0, c_hi = WIDE ? min(n64, eh * 2 + 2) : n64;
                 if (c_lo >= c_hi) release();
-                for (int c = c_lo; c < c_hi; ++c) {
+                // one piece: 64 slots from column 64 c on, lane group gs
+                auto finish_piece = [&](int c, int gs, uint32_t (&o)[8]) {
+                    uint32_t v[32];
+                    tmem_ld_16x64(taddr + ((uint32_t)(gs * 16) << 16) + (uint32_t)(c * 64), v);
 #pragma unroll
-                    for (int gs = 0; gs < 2; ++gs) {
-                        uint32_t v[32];
-                        tmem_ld_16x64(taddr + ((uint32_t)(gs * 16) << 16) + (uint32_t)(c * 64), v);
-                        if (c == c_hi - 1 && gs == 1) release();
-                        uint32_t o[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            float g0 = __uint_as_float(v[4 * j]), g1 = __uint_as_float(v[4 * j + 1]);
-                            float u0 = __uint_as_float(v[4 * j + 2]), u1 = __uint_as_float(v[4 * j + 3]);
-                            if (!AFFINE || TWO) { g0 *= rf[2 * gs]; g1 *= rf[2 * gs]; u0 *= rf[2 * gs + 1]; u1 *= rf[2 * gs + 1]; }
-                            const float r0 = silu_fast(g0) * u0, r1 = silu_fast(g1) * u1;
-                            peak = fmaxf(peak, fmaxf(fabsf(r0), fabsf(r1)));
-                            o[j] = pack_f16_sat(r0, r1);
-                        }
-                        const int col = t.ntile * 64 + (2 * q + gs) * 8 + (lane >> 2);
-                        const int pos = (col & ~15) + (int)((p.pos_lut >> (4 * (col & 15))) & 0xf);
-                        const int sl0 = c * 64 + 2 * (lane & 3);                 // first of this thread's slots
-                        __half* dst = a.act + (size_t)(t.slot0 + sl0) * a.act_stride + pos;
-                        const int n_ok = t.rows - sl0;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            if (8 * j < n_ok) st_global_u16(dst + (size_t)(8 * j) * a.act_stride, o[j]);
-                            if (8 * j + 1 < n_ok) st_global_u16(dst + (size_t)(8 * j + 1) * a.act_stride, o[j] >> 16);
-                        }
+                    for (int j = 0; j < 8; ++j) {
+                        float g0 = __uint_as_float(v[4 * j]), g1 = __uint_as_float(v[4 * j + 1]);
+                        float u0 = __uint_as_float(v[4 * j + 2]), u1 = __uint_as_float(v[4 * j + 3]);
+                        if (!AFFINE || TWO) { g0 *= rf[2 * gs]; g1 *= rf[2 * gs]; u0 *= rf[2 * gs + 1]; u1 *= rf[2 * gs + 1]; }
+                        const float r0 = silu_fast(g0) * u0, r1 = silu_fast(g1) * u1;
+                        peak = fmaxf(peak, fmaxf(fabsf(r0), fabsf(r1)));
+                        o[j] = pack_f16_sat(r0, r1);
                     }
+                };
+                auto store_piece = [&](int c, int gs, const uint32_t (&o)[8]) {
+                    const int col = t.ntile * 64 + (2 * q + gs) * 8 + (lane >> 2);
+                    const int pos = (col & ~15) + (int)((p.pos_lut >> (4 * (col & 15))) & 0xf);
+                    const int sl0 = c * 64 + 2 * (lane & 3);                 // first of this thread's slots
+                    __half* dst = a.act + (size_t)(t.slot0 + sl0) * a.act_stride + pos;
+                    const int n_ok = t.rows - sl0;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (8 * j < n_ok) st_global_u16(dst + (size_t)(8 * j) * a.act_stride, o[j]);
+                        if (8 * j + 1 < n_ok) st_global_u16(dst + (size_t)(8 * j + 1) * a.act_stride, o[j] >> 16);
+                    }
+                };
+                if (WIDE) {
+                    // everything leaves tensor memory before the first store: the accumulator is free that much earlier
+                    uint32_t o[2][2][8];
+#pragma unroll
+                    for (int cc = 0; cc < 2; ++cc)
+                        if (c_lo + cc < c_hi) {
+                            finish_piece(c_lo + cc, 0, o[cc][0]);
+                            finish_piece(c_lo + cc, 1, o[cc][1]);
+                        }
+                    if (c_lo < c_hi) release();
+#pragma unroll
+                    for (int cc = 0; cc < 2; ++cc)
+                        if (c_lo + cc < c_hi) {
+                            store_piece(c_lo + cc, 0, o[cc][0]);
+                            store_piece(c_lo + cc, 1, o[cc][1]);
+                        }
+                } else {
+                    for (int c = c_lo; c < c_hi; ++c)
+#pragma unroll
+                        for (int gs = 0; gs < 2; ++gs) {
+                            uint32_t o[8];
+                            finish_piece(c, gs, o);
+                            if (c == c_hi - 1 && gs == 1) release();
+                            store_piece(c, gs, o);
+                        }
                 }
             } else {
                 const int chunks = (t.rows + 31) >> 5;
                 const int c_lo = WIDE ? eh * 4 : 0, c_hi = WIDE ? min(chunks, eh * 4 + 4) : chunks;
                 if (c_lo >= c_hi) release();
                 const int col = t.ntile * 128 + lane128;
+                if (WIDE && c_lo < c_hi && a.row_scale == nullptr && a.out_index == nullptr && a.out16 != nullptr) {
+                    // All of the warp's columns leave tensor memory as packed pairs before the first is stored: the
+                    // single accumulator is free for the next tile's MMAs that much earlier (a 512-long reduction is
+                    // eight K steps, a quarter of its time went by while the rows were written).
+                    uint32_t h[4][16];
+#pragma unroll
+                    for (int cc = 0; cc < 4; ++cc) {
+                        if (c_lo + cc < c_hi) {
+                            uint32_t v[32];
+                            tmem_ld32(taddr + (c_lo + cc) * 32, v);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) {
+                                float x0 = __uint_as_float(v[2 * i]), x1 = __uint_as_float(v[2 * i + 1]);
+                                if (!AFFINE || TWO) { x0 *= rf[0]; x1 *= rf[0]; }
+                                peak = fmaxf(peak, fmaxf(fabsf(x0), fabsf(x1)));
+                                h[cc][i] = pack_f16_sat(x0, x1);
+                            }
+                        }
+                    }
+                    release();
+#pragma unroll
+                    for (int cc = 0; cc < 4; ++cc) {
+                        __half* dst = a.out16 + (size_t)(t.slot0 + (c_lo + cc) * 32) * a.set.n_in + col;
+                        const int n_ok = t.rows - (c_lo + cc) * 32;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            if (2 * i < n_ok) st_global_u16(dst + (size_t)(2 * i) * a.set.n_in, h[cc][i]);
+                            if (2 * i + 1 < n_ok) st_global_u16(dst + (size_t)(2 * i + 1) * a.set.n_in, h[cc][i] >> 16);
+                        }
+                    }
+                } else
                 for (int c = c_lo; c < c_hi; ++c) {
                     uint32_t v[32];
                     tmem_ld32(taddr + c * 32, v);
@@ -936,7 +1071,7 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
         Ring r = {0, 0u};
         r.advance(grp_id, stages);
         PROF_DECL
-        for_each_tile<SWIGLU, XR, SPLIT>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
+        for_each_tile<SWIGLU, XR, SPLIT, PAIR>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
             const int ksteps = t.K / kTileK;
             const int sbuf = it & 1;
             const uint32_t srow = (uint32_t)(t.K >> p.lg_group) * (AFFINE ? 2u : 1u);
@@ -1039,7 +1174,10 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
                     fence_async_proxy();                 // generic-proxy writes -> visible to the tensor-core reads
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->full[r.s]));
+                if (lane == 0) {
+                    if (PAIR) mbar_arrive_cta0(smem_u32(&bars->full[r.s]));
+                    else mbar_arrive(smem_u32(&bars->full[r.s]));
+                }
                 PROF_END(2)
                 r.advance(2, stages);
             }
@@ -1057,10 +1195,24 @@ prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__
 
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();                                // neither CTA leaves while the other may arrive on its barriers
     if (warp == 1) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     }
     if (tid == 0 && bars->abort && a.status != nullptr) atomicExch(a.status, 3);
+}
+
+template <bool SWIGLU, int FMT, bool TS, bool WIDE, bool XR>
+__global__ void __launch_bounds__(kThreadsTc, 1)
+prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__ TcMaps maps) {
+    prefill_tc_body<SWIGLU, FMT, TS, WIDE, XR, false>(a, p, maps);
+}
+
+template <bool SWIGLU, int FMT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsTc, 1)
+prefill_pair_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__ TcMaps maps) {
+    prefill_tc_body<SWIGLU, FMT, true, true, false, true>(a, p, maps);
 }
 
 }  // namespace
@@ -1115,6 +1267,8 @@ constexpr size_t kSmemMost = 227 * 1024;
 template <int FMT>
 int configure() {
     constexpr int kSmem = (int)kSmemMost;
+    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_pair_kernel<true, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_pair_kernel<false, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     if constexpr (two_term(FMT)) {
         IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
         IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
@@ -1135,6 +1289,7 @@ struct Plan {
     TcParams p;
     size_t smem;
     bool wide;
+    bool pair;
     bool xr;
 };
 
@@ -1143,25 +1298,29 @@ int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, co
                cudaStream_t stream, cudaEvent_t mid) {
     if constexpr (two_term(FMT)) {
         if (!a.second_only) {
-            prefill_tc_kernel<true, FMT, true, true, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+            if (gu.pair) prefill_pair_kernel<true, FMT><<<sms & ~1, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+            else prefill_tc_kernel<true, FMT, true, true, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
             IMX_LAUNCHED();
             IMX_CHECK_CUDA(cudaGetLastError());
         }
         if (mid) IMX_CHECK_CUDA(cudaEventRecord(mid, stream));
-        prefill_tc_kernel<false, FMT, true, true, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        if (dn.pair) prefill_pair_kernel<false, FMT><<<sms & ~1, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        else prefill_tc_kernel<false, FMT, true, true, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
         IMX_LAUNCHED();
         IMX_CHECK_CUDA(cudaGetLastError());
         return IMX_OK;
     } else {
     if (!a.second_only) {
-        if (!ts) prefill_tc_kernel<true, FMT, false, false, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+        if (gu.pair) prefill_pair_kernel<true, FMT><<<sms & ~1, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+        else if (!ts) prefill_tc_kernel<true, FMT, false, false, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
         else if (gu.wide) prefill_tc_kernel<true, FMT, true, true, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
         else prefill_tc_kernel<true, FMT, true, false, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
         IMX_LAUNCHED();
         IMX_CHECK_CUDA(cudaGetLastError());
     }
     if (mid) IMX_CHECK_CUDA(cudaEventRecord(mid, stream));
-    if (!ts) prefill_tc_kernel<false, FMT, false, false, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+    if (dn.pair) prefill_pair_kernel<false, FMT><<<sms & ~1, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+    else if (!ts) prefill_tc_kernel<false, FMT, false, false, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
     else if (dn.wide) prefill_tc_kernel<false, FMT, true, true, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
     else if (dn.xr) prefill_tc_kernel<false, FMT, true, false, true><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
     else prefill_tc_kernel<false, FMT, true, false, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
@@ -1174,11 +1333,11 @@ int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, co
 // Shared memory of a launch: [panel][stages][two scale buffers][control block].  As many stages as fit,
 // at most 8 (4 with two-term weights: the ring of A tiles in tensor memory has 256 columns) and, with a resident
 // panel, at most the shortest reduction's K steps (the ring's back-pressure then also guards the panel).
-bool make_plan(const QFormat& f, int fmt, int K_max, int K_min, bool wide, bool xr, bool ts, Plan* out) {
+bool make_plan(const QFormat& f, int fmt, int K_max, int K_min, bool wide, bool xr, bool ts, Plan* out, bool pair = false) {
     const size_t q_tile = 128u * (size_t)q_row_bytes(fmt);
     const size_t sc = (size_t)128 * scale_row(K_max, f) * (f.mode == IMX_MODE_AFFINE ? 2 : 1);
     const size_t panel = xr ? (size_t)(K_max / kTileK) * kXBytes : 0;
-    const size_t stage = (xr ? 0 : (size_t)kXBytes * (wide ? 2 : 1) + (ts ? 0 : kWBytes)) + q_tile;
+    const size_t stage = (xr ? 0 : (size_t)kXBytes * (wide && !pair ? 2 : 1) + (ts ? 0 : kWBytes)) + q_tile;
     const size_t fixed = panel + 2 * sc + sizeof(Bars) + 1024;
     if (fixed + 2 * stage > kSmemMost) return false;
     int st = (int)((kSmemMost - fixed) / stage);
@@ -1194,6 +1353,7 @@ bool make_plan(const QFormat& f, int fmt, int K_max, int K_min, bool wide, bool 
     out->p.lg_group = log2_exact(f.group);
     out->smem = fixed + (size_t)st * stage;
     out->wide = wide;
+    out->pair = pair;
     out->xr = xr;
     return true;
 }
@@ -1300,6 +1460,11 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
     if (!(variant == 0 && (plan(mid_max, mid_min, true, false, &dn) || plan(mid_max, mid_min, false, true, &dn))))
         IMX_REQUIRE(plan(mid_max, mid_min, false, false, &dn), "prefill path: sizes exceed shared memory");
     }
+    // wide tiles in pairs of CTAs wherever the weight tiles of a unit pair up
+    if (gu.wide && s.n_mid % 128 == 0 && x_mid % 128 == 0)
+        IMX_REQUIRE(make_plan(f, fmt, s.n_in, s.n_in, true, false, true, &gu, true), "prefill path: sizes exceed shared memory");
+    if (dn.wide && s.n_in % 256 == 0)
+        IMX_REQUIRE(make_plan(f, fmt, mid_max, mid_min, true, false, true, &dn, true), "prefill path: sizes exceed shared memory");
     gu.p.nt_r = s.n_mid / 64;
     gu.p.nt_x = x_mid / 64;
     dn.p.nt_r = dn.p.nt_x = s.n_in / 128;
