@@ -123,7 +123,8 @@ struct TcParams {
     int sc_bytes;                                  // one tile's scale buffer
     int panel_bytes;                               // resident activation panel (0: streamed per stage)
     int lg_group;                                  // log2 of the group size
-    unsigned long long pos_lut;                    // position of reduction index i inside its block of 16, 4 bits each
+    int epi_bytes;                                 // wide tiles: the epilogue warps' transposing buffers
+    unsigned long long ord_lut;                    // reduction index at position p of a block of 16, 4 bits each
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -283,6 +284,18 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// Four (two) 8 x 8 matrices of 16-bit values in the MMA fragment layout (thread t: row t / 4, columns 2 (t % 4), + 1) to
+// shared memory, transposed: lane 8 m + i names the 16 bytes column i of matrix m goes to.
+__device__ __forceinline__ void stmatrix4_trans(uint32_t addr, uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(m0), "r"(m1), "r"(m2), "r"(m3)
+                 : "memory");
+}
+__device__ __forceinline__ void stmatrix2_trans(uint32_t addr, uint32_t m0, uint32_t m1) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x2.trans.shared.b16 [%0], {%1, %2};" ::"r"(addr), "r"(m0), "r"(m1) : "memory");
+}
+__device__ __forceinline__ void st_global_128(void* p, uint4 v) {
+    asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
@@ -421,12 +434,15 @@ __device__ __forceinline__ void tile_rows(const GroupedArgs& a, const TileInfo& 
 // Row of the 128-row tile (0..127: the order of the two TMA boxes: first product 64 gate rows, then the 64
 // matching up rows) a tensor-memory lane holds.  First product: in every group of 16 lanes the first 8 hold
 // gate rows and the other 8 the matching up rows, so that a 16-lane tensor-memory load hands a thread the gate
-// and the up value of the same (row, slot) and SwiGLU needs no exchange between threads.
+// and the up value of the same (row, slot) and SwiGLU needs no exchange between threads.  The 16 rows of two
+// groups are a block of 16 output columns, taken in the order their values are stored in (ord_lut: the order the
+// second product's weights are unpacked in), so that neighbouring lanes write neighbouring values.
 template <bool SWIGLU>
-__device__ __forceinline__ int tile_row_of_lane(int lane128) {
+__device__ __forceinline__ int tile_row_of_lane(int lane128, unsigned long long ord_lut) {
     if (!SWIGLU) return lane128;
     const int grp = lane128 >> 4, w = lane128 & 15;
-    return ((w >> 3) << 6) + grp * 8 + (w & 7);
+    const int at = (grp & 1) * 8 + (w & 7);
+    return ((w >> 3) << 6) + (grp >> 1) * 16 + (int)((ord_lut >> (4 * at)) & 0xf);
 }
 
 // ── dequantization of one weight row's K step: 64 values -> 32 registers of fp16 pairs ──
@@ -702,8 +718,8 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
     constexpr bool SPLIT = !WIDE;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    // [activation panel (XR)][stages][2 tiles' scale buffers][control block]
-    Bars* bars = reinterpret_cast<Bars*>(base + (size_t)p.panel_bytes + (size_t)p.stages * p.stage_bytes + 2 * (size_t)p.sc_bytes);
+    // [activation panel (XR)][stages][2 tiles' scale buffers][transposing buffers (WIDE)][control block]
+    Bars* bars = reinterpret_cast<Bars*>(base + (size_t)p.panel_bytes + (size_t)p.stages * p.stage_bytes + 2 * (size_t)p.sc_bytes + p.epi_bytes);
     const uint32_t panel = smem_u32(base);
     const uint32_t sbase = panel + (uint32_t)p.panel_bytes;
     const uint32_t sc_base = sbase + (uint32_t)(p.stages * p.stage_bytes);
@@ -855,6 +871,10 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
         const int q = warp & 3;                                 // tensor-memory lane quarter
         const int eh = warp >= 16 ? 1 : 0;                      // WIDE: which half of the tile's slots; else: which accumulator
         const int lane128 = q * 32 + lane;
+        // this warp's transposing buffer: 64 slots of 32 (second product: 64) bytes, rows padded so that eight of them
+        // spread over all banks
+        constexpr uint32_t kEpiRow = SWIGLU ? 48 : 80;
+        const uint32_t ebuf = sc_base + 2u * (uint32_t)p.sc_bytes + (uint32_t)(eh * 4 + q) * 64u * kEpiRow;
         PROF_DECL
         for_each_tile<SWIGLU, XR, SPLIT, PAIR>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
             const int buf = it % NB, round = it / NB;
@@ -882,14 +902,21 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                 for (int i = 0; i < srow; i += 16) mx = max_byte(__ldg(reinterpret_cast<const uint4*>(sp + i)), mx);
                 return ue8m0_to_f32(hmax_bytes(mx));
             };
-            float rf[4] = {1.f, 1.f, 1.f, 1.f};                     // first product: [lane group][gate, up]; second: [0]
+            // [lane group of 16][gate, up], or the weight rows 16 gs + 8 r8 + lane / 4 of the warp's 32; second product
+            // with one weight row a lane (fp32 rows): [0]
+            float rf[4] = {1.f, 1.f, 1.f, 1.f};
+            const bool frag_rows = !SWIGLU && WIDE && a.row_scale == nullptr && a.out16 != nullptr;
             if (SWIGLU) {
 #pragma unroll
                 for (int gs = 0; gs < 2; ++gs) {
-                    const int idx = t.ntile * 64 + (2 * q + gs) * 8 + (lane >> 2);
+                    const int idx = t.ntile * 64 + q * 16 + (int)((p.ord_lut >> (4 * (gs * 8 + (lane >> 2)))) & 0xf);
                     rf[2 * gs] = row_factor(t.extra ? S.x_gate : S.gate, S.gu_stride_s, idx);
                     rf[2 * gs + 1] = row_factor(t.extra ? S.x_up : S.up, S.gu_stride_s, idx);
                 }
+            } else if (frag_rows) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    rf[i] = row_factor(t.extra ? S.x_down : S.down, S.dn_stride_s, t.ntile * 128 + q * 32 + i * 8 + (lane >> 2));
             } else {
                 rf[0] = row_factor(t.extra ? S.x_down : S.down, S.dn_stride_s, t.ntile * 128 + lane128);
             }
@@ -915,7 +942,9 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                 const int c_lo = WIDE ? eh * 2 : 0, c_hi = WIDE ? min(n64, eh * 2 + 2) : n64;
                 if (c_lo >= c_hi) release();
                 // one piece: 64 slots from column 64 c on, lane group gs
+                // (columns past the unit's rows hold what earlier tiles left: they are not counted as clamped)
                 auto finish_piece = [&](int c, int gs, uint32_t (&o)[8]) {
+                    const int n_ok = t.rows - c * 64 - 2 * (lane & 3);
                     uint32_t v[32];
                     tmem_ld_16x64(taddr + ((uint32_t)(gs * 16) << 16) + (uint32_t)(c * 64), v);
 #pragma unroll
@@ -924,15 +953,14 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                         float u0 = __uint_as_float(v[4 * j + 2]), u1 = __uint_as_float(v[4 * j + 3]);
                         if (!AFFINE || TWO) { g0 *= rf[2 * gs]; g1 *= rf[2 * gs]; u0 *= rf[2 * gs + 1]; u1 *= rf[2 * gs + 1]; }
                         const float r0 = silu_fast(g0) * u0, r1 = silu_fast(g1) * u1;
-                        peak = fmaxf(peak, fmaxf(fabsf(r0), fabsf(r1)));
+                        peak = fmaxf(peak, fmaxf(8 * j < n_ok ? fabsf(r0) : 0.f, 8 * j + 1 < n_ok ? fabsf(r1) : 0.f));
                         o[j] = pack_f16_sat(r0, r1);
                     }
                 };
+                const int pos0 = t.ntile * 64 + q * 16;                      // first of the warp's 16 stored columns
                 auto store_piece = [&](int c, int gs, const uint32_t (&o)[8]) {
-                    const int col = t.ntile * 64 + (2 * q + gs) * 8 + (lane >> 2);
-                    const int pos = (col & ~15) + (int)((p.pos_lut >> (4 * (col & 15))) & 0xf);
                     const int sl0 = c * 64 + 2 * (lane & 3);                 // first of this thread's slots
-                    __half* dst = a.act + (size_t)(t.slot0 + sl0) * a.act_stride + pos;
+                    __half* dst = a.act + (size_t)(t.slot0 + sl0) * a.act_stride + pos0 + gs * 8 + (lane >> 2);
                     const int n_ok = t.rows - sl0;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
@@ -953,8 +981,21 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
 #pragma unroll
                     for (int cc = 0; cc < 2; ++cc)
                         if (c_lo + cc < c_hi) {
-                            store_piece(c_lo + cc, 0, o[cc][0]);
-                            store_piece(c_lo + cc, 1, o[cc][1]);
+                            // 64 slots x 16 columns, turned round in shared memory: a slot's 32 bytes go out as two
+                            // 16-byte stores, 16 slots at a time, instead of as single values
+                            const uint32_t at = ebuf + (uint32_t)(lane & 7) * kEpiRow + (uint32_t)((lane >> 3) & 1) * 16u;
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) stmatrix2_trans(at + (uint32_t)j * 8u * kEpiRow, o[cc][0][j], o[cc][1][j]);
+                            __syncwarp();
+                            const int sl0 = (c_lo + cc) * 64;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const int sl = i * 16 + (lane >> 1);
+                                const uint4 v = lds128(ebuf + (uint32_t)sl * kEpiRow + (uint32_t)(lane & 1) * 16u);
+                                if (sl0 + sl < t.rows)
+                                    st_global_128(a.act + (size_t)(t.slot0 + sl0 + sl) * a.act_stride + pos0 + (lane & 1) * 8, v);
+                            }
+                            __syncwarp();
                         }
                 } else {
                     for (int c = c_lo; c < c_hi; ++c)
@@ -971,35 +1012,64 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                 const int c_lo = WIDE ? eh * 4 : 0, c_hi = WIDE ? min(chunks, eh * 4 + 4) : chunks;
                 if (c_lo >= c_hi) release();
                 const int col = t.ntile * 128 + lane128;
-                if (WIDE && c_lo < c_hi && a.row_scale == nullptr && a.out_index == nullptr && a.out16 != nullptr) {
+                if (frag_rows && c_lo < c_hi) {
                     // All of the warp's columns leave tensor memory as packed pairs before the first is stored: the
-                    // single accumulator is free for the next tile's MMAs that much earlier (a 512-long reduction is
-                    // eight K steps, a quarter of its time went by while the rows were written).
-                    uint32_t h[4][16];
+                    // single accumulator is free for the next tile's MMAs that much earlier.  Then 64 slots x 32
+                    // columns at a time are turned round in shared memory and go out as 16-byte pieces, 8 slots an
+                    // instruction.  As single values, 64 bytes an instruction, the stores of a tile took longer than
+                    // the MMAs of a 512-long reduction (role times of CTA 0, 8192 tokens: epilogue busy 274 of 357
+                    // thousand cycles); the block went from 833 to 793 us.
+                    const int n64 = (t.rows - eh * 128 + 63) >> 6;  // pieces of 64 slots of this warp's half: 1 or 2
+                    // a piece as fragments: [8 weight rows][8 slots]
+                    auto drain = [&](int c, uint32_t (&h)[4][8]) {
+                        const int n_ok = t.rows - (eh * 2 + c) * 64 - 2 * (lane & 3);
 #pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) {
-                        if (c_lo + cc < c_hi) {
+                        for (int gs = 0; gs < 2; ++gs) {
                             uint32_t v[32];
-                            tmem_ld32(taddr + (c_lo + cc) * 32, v);
+                            tmem_ld_16x64(taddr + ((uint32_t)(gs * 16) << 16) + (uint32_t)((eh * 2 + c) * 64), v);
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                float x0 = __uint_as_float(v[2 * i]), x1 = __uint_as_float(v[2 * i + 1]);
-                                if (!AFFINE || TWO) { x0 *= rf[0]; x1 *= rf[0]; }
-                                peak = fmaxf(peak, fmaxf(fabsf(x0), fabsf(x1)));
-                                h[cc][i] = pack_f16_sat(x0, x1);
+                            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                                for (int r8 = 0; r8 < 2; ++r8) {
+                                    float x0 = __uint_as_float(v[4 * j + 2 * r8]), x1 = __uint_as_float(v[4 * j + 2 * r8 + 1]);
+                                    if (!AFFINE || TWO) { x0 *= rf[2 * gs + r8]; x1 *= rf[2 * gs + r8]; }
+                                    peak = fmaxf(peak, fmaxf(8 * j < n_ok ? fabsf(x0) : 0.f, 8 * j + 1 < n_ok ? fabsf(x1) : 0.f));
+                                    h[2 * gs + r8][j] = pack_f16_sat(x0, x1);
+                                }
+                        }
+                    };
+                    auto turn = [&](const uint32_t (&h)[4][8]) {
+                        const uint32_t at = ebuf + (uint32_t)(lane & 7) * kEpiRow + (uint32_t)(lane >> 3) * 16u;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) stmatrix4_trans(at + (uint32_t)j * 8u * kEpiRow, h[0][j], h[1][j], h[2][j], h[3][j]);
+                        __syncwarp();
+                    };
+                    auto flush = [&](int c) {
+                        const int sl0 = (eh * 2 + c) * 64;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int sl = i * 8 + (lane >> 2);
+                            const uint4 v = lds128(ebuf + (uint32_t)sl * kEpiRow + (uint32_t)(lane & 3) * 16u);
+                            if (sl0 + sl < t.rows) {
+                                const int slot = t.slot0 + sl0 + sl;
+                                const int orow = a.out_index != nullptr ? a.out_index[slot] : slot;
+                                st_global_128(a.out16 + (size_t)orow * a.set.n_in + t.ntile * 128 + q * 32 + (lane & 3) * 8, v);
                             }
                         }
+                        __syncwarp();
+                    };
+                    uint32_t h[4][8];
+                    drain(0, h);
+                    if (n64 == 1) release();
+                    turn(h);
+                    if (n64 > 1) {
+                        drain(1, h);
+                        release();
                     }
-                    release();
-#pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) {
-                        __half* dst = a.out16 + (size_t)(t.slot0 + (c_lo + cc) * 32) * a.set.n_in + col;
-                        const int n_ok = t.rows - (c_lo + cc) * 32;
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            if (2 * i < n_ok) st_global_u16(dst + (size_t)(2 * i) * a.set.n_in, h[cc][i]);
-                            if (2 * i + 1 < n_ok) st_global_u16(dst + (size_t)(2 * i + 1) * a.set.n_in, h[cc][i] >> 16);
-                        }
+                    flush(0);
+                    if (n64 > 1) {
+                        turn(h);
+                        flush(1);
                     }
                 } else
                 for (int c = c_lo; c < c_hi; ++c) {
@@ -1062,7 +1132,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
         // two groups of four warps on alternating K steps; a thread owns one weight row of the tile
         const int grp_id = (warp - 8) >> 2;
         const int lane128 = tid - 256 - grp_id * 128;     // tensor-memory lane = (warp % 4) * 32 + lane
-        const int qrow = tile_row_of_lane<SWIGLU>(lane128);
+        const int qrow = tile_row_of_lane<SWIGLU>(lane128, p.ord_lut);
         const uint32_t swz = QROW == 32 ? ((uint32_t)qrow >> 2) & 1u : (QROW == 64 ? ((uint32_t)qrow >> 1) & 3u : 0u);
         const uint32_t q_off = Q_OFF + (uint32_t)qrow * QROW;
         const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + kTmemA;
@@ -1333,12 +1403,13 @@ int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, co
 // Shared memory of a launch: [panel][stages][two scale buffers][control block].  As many stages as fit,
 // at most 8 (4 with two-term weights: the ring of A tiles in tensor memory has 256 columns) and, with a resident
 // panel, at most the shortest reduction's K steps (the ring's back-pressure then also guards the panel).
-bool make_plan(const QFormat& f, int fmt, int K_max, int K_min, bool wide, bool xr, bool ts, Plan* out, bool pair = false) {
+bool make_plan(const QFormat& f, int fmt, int K_max, int K_min, bool wide, bool xr, bool ts, Plan* out, bool pair = false, int epi_row = 0) {
     const size_t q_tile = 128u * (size_t)q_row_bytes(fmt);
     const size_t sc = (size_t)128 * scale_row(K_max, f) * (f.mode == IMX_MODE_AFFINE ? 2 : 1);
     const size_t panel = xr ? (size_t)(K_max / kTileK) * kXBytes : 0;
     const size_t stage = (xr ? 0 : (size_t)kXBytes * (wide && !pair ? 2 : 1) + (ts ? 0 : kWBytes)) + q_tile;
-    const size_t fixed = panel + 2 * sc + sizeof(Bars) + 1024;
+    const size_t epi = wide ? (size_t)8 * 64 * (size_t)epi_row : 0;
+    const size_t fixed = panel + 2 * sc + epi + sizeof(Bars) + 1024;
     if (fixed + 2 * stage > kSmemMost) return false;
     int st = (int)((kSmemMost - fixed) / stage);
     const int most = two_term(fmt) ? 4 : kMaxStages;
@@ -1350,12 +1421,21 @@ bool make_plan(const QFormat& f, int fmt, int K_max, int K_min, bool wide, bool 
     out->p.stage_bytes = (int)stage;
     out->p.sc_bytes = (int)sc;
     out->p.panel_bytes = (int)panel;
+    out->p.epi_bytes = (int)epi;
     out->p.lg_group = log2_exact(f.group);
     out->smem = fixed + (size_t)st * stage;
     out->wide = wide;
     out->pair = pair;
     out->xr = xr;
     return true;
+}
+
+// Wide tiles of one product: in pairs of CTAs where the weight tiles of a unit pair up, else one CTA each.  16-bit
+// results are turned round in shared memory (first product 48, second 80 bytes a slot; fp32 rows need none).
+constexpr int kEpiFirst = 48, kEpiSecond = 80;
+bool wide_plan(const QFormat& f, int fmt, int K_max, int K_min, bool even, int epi_row, Plan* out) {
+    return (even && make_plan(f, fmt, K_max, K_min, true, false, true, out, true, epi_row)) ||
+           make_plan(f, fmt, K_max, K_min, true, false, true, out, false, epi_row);
 }
 
 }  // namespace
@@ -1392,6 +1472,10 @@ void two_term_block_order(int bits, int order[16]) {
     else two_term_order<4>(order);
 }
 
+// Do the weight tiles of a unit pair up (64 gate and 64 up rows, 128 output rows a tile)?
+static bool first_even(const ExpertSet& s) { return s.n_mid % 128 == 0 && (!s.has_extra || s.x_mid % 128 == 0); }
+static bool second_even(const ExpertSet& s) { return s.n_in % 256 == 0; }
+
 bool two_term_supported(const ExpertSet& s, bool second_only) {
     const QFormat& f = s.fmt;
     const int fmt = two_term_index(f);
@@ -1402,8 +1486,8 @@ bool two_term_supported(const ExpertSet& s, bool second_only) {
     if ((!second_only && !ok(s.n_in)) || !ok(s.n_mid) || (s.has_extra && !ok(s.x_mid))) return false;
     const int mid_max = s.has_extra && s.x_mid > s.n_mid ? s.x_mid : s.n_mid;
     Plan p;
-    return (second_only || make_plan(f, fmt, s.n_in, s.n_in, true, false, true, &p)) &&
-           make_plan(f, fmt, mid_max, mid_max, true, false, true, &p);
+    return (second_only || wide_plan(f, fmt, s.n_in, s.n_in, first_even(s), kEpiFirst, &p)) &&
+           wide_plan(f, fmt, mid_max, mid_max, second_even(s), 0, &p);
 }
 
 // What the copy engine asks of the matrices' addresses (the scalar kernel takes any 16 / 4-byte aligned tensor).
@@ -1449,32 +1533,29 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
         return make_plan(f, fmt, K_max, K_min, wide, xr, ts, out);
     };
     Plan gu = {}, dn = {};
+    const int epi_second = a.out16 != nullptr ? kEpiSecond : 0;
     if (variant == 3) {
-        IMX_REQUIRE((a.second_only || plan(s.n_in, s.n_in, true, false, &gu)) && plan(mid_max, mid_min, true, false, &dn),
+        IMX_REQUIRE((a.second_only || wide_plan(f, fmt, s.n_in, s.n_in, first_even(s), kEpiFirst, &gu)) &&
+                        wide_plan(f, fmt, mid_max, mid_min, second_even(s), epi_second, &dn),
                     "two-term path: sizes exceed shared memory");
     } else {
-    if (!a.second_only && !(variant == 0 && plan(s.n_in, s.n_in, true, false, &gu)))
-        IMX_REQUIRE(plan(s.n_in, s.n_in, false, false, &gu), "prefill path: sizes exceed shared memory");
-    // second product: 256-slot tiles with streamed activations as well (c3: 276 us against 377 us with 128-slot
-    // tiles and the activation panel resident); the resident panel where the wide stages do not fit
-    if (!(variant == 0 && (plan(mid_max, mid_min, true, false, &dn) || plan(mid_max, mid_min, false, true, &dn))))
-        IMX_REQUIRE(plan(mid_max, mid_min, false, false, &dn), "prefill path: sizes exceed shared memory");
+        if (!a.second_only && !(variant == 0 && wide_plan(f, fmt, s.n_in, s.n_in, first_even(s), kEpiFirst, &gu)))
+            IMX_REQUIRE(plan(s.n_in, s.n_in, false, false, &gu), "prefill path: sizes exceed shared memory");
+        // second product: 256-slot tiles with streamed activations as well (c3: 276 us against 377 us with 128-slot
+        // tiles and the activation panel resident, one CTA a tile); the resident panel where the wide stages do not fit
+        if (!(variant == 0 && (wide_plan(f, fmt, mid_max, mid_min, second_even(s), epi_second, &dn) || plan(mid_max, mid_min, false, true, &dn))))
+            IMX_REQUIRE(plan(mid_max, mid_min, false, false, &dn), "prefill path: sizes exceed shared memory");
     }
-    // wide tiles in pairs of CTAs wherever the weight tiles of a unit pair up
-    if (gu.wide && s.n_mid % 128 == 0 && x_mid % 128 == 0)
-        IMX_REQUIRE(make_plan(f, fmt, s.n_in, s.n_in, true, false, true, &gu, true), "prefill path: sizes exceed shared memory");
-    if (dn.wide && s.n_in % 256 == 0)
-        IMX_REQUIRE(make_plan(f, fmt, mid_max, mid_min, true, false, true, &dn, true), "prefill path: sizes exceed shared memory");
     gu.p.nt_r = s.n_mid / 64;
     gu.p.nt_x = x_mid / 64;
     dn.p.nt_r = dn.p.nt_x = s.n_in / 128;
-    // where the first product's epilogue puts output column i of a block of 16: the order the second
-    // product's weights are unpacked in
+    // the order of a block of 16 the first product's epilogue writes: the one the second product's weights are
+    // unpacked in
     int order[16];
     expert_block_order(f, order);
     unsigned long long lut = 0;
-    for (int pos = 0; pos < 16; ++pos) lut |= (unsigned long long)pos << (4 * order[pos]);
-    gu.p.pos_lut = dn.p.pos_lut = lut;
+    for (int pos = 0; pos < 16; ++pos) lut |= (unsigned long long)order[pos] << (4 * pos);
+    gu.p.ord_lut = dn.p.ord_lut = lut;
 
     // activations in sorted-slot order (the `take_axis` of moe.rs:124-127, once for all experts)
     const __half* xsrc = a.in;                     // already slot-ordered when there is no row index
