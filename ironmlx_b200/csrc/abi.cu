@@ -362,7 +362,7 @@ static int forward_impl(const imx_moe_config* cfg, const imx_moe_weights* w, con
     IMX_TRY(launch_route(router_in, n_tokens, c.hidden, w->router_w, w->router_logit_bias, c.num_experts, c.top_k,
                          c.norm_topk_prob, has_shared ? w->shared_expert_gate_w : nullptr, ws.topk_idx,
                          ws.topk_w, ws.shared_gate, ws.x16, order, stream,
-                         tmap_decode ? 0.0625f : 1.f, ws.route_partials ? &rscratch : nullptr, &sums_done));
+                         tmap_decode ? 0.0625f : 1.f, ws.route_partials ? &rscratch : nullptr, &sums_done, ws.status));
     IMX_CHECK_CUDA(mark(1));
     SortExtras ex;
     ex.topk_w = ws.topk_w;

@@ -74,6 +74,31 @@ struct Codec<2> {
     }
 };
 
+// The widths that do not divide a word: codes are pulled out of the bit stream in pairs (a, a + D) (what D is for, see
+// the two-term weights of the tensor-core kernels); codes of a block of 16 without a partner at that distance pair with
+// their neighbour (6-bit: (12, 15) and (13, 14)).
+template <int BITS>
+struct PairOrder {
+    static constexpr int D = BITS == 3 ? 6 : (BITS == 6 ? 3 : 4);
+    static constexpr int SPAN = BITS == 3 ? 12 : (BITS == 6 ? 6 : 8);   // codes that pair up among themselves
+    // first code of pair p of a block of 16 and the distance of its partner
+    __host__ __device__ static constexpr int first(int p) {
+        const int full = 16 / SPAN * SPAN, rest = p - full / 2;
+        if (rest < 0) return p / D * SPAN + p % D;
+        if (BITS == 6) return rest == 0 ? 12 : 13;
+        return full + 2 * rest;
+    }
+    __host__ __device__ static constexpr int dist(int p) {
+        const int full = 16 / SPAN * SPAN, rest = p - full / 2;
+        if (rest < 0) return D;
+        return BITS == 6 && rest == 0 ? 3 : 1;
+    }
+    __host__ __device__ static constexpr int order(int p) { return first(p >> 1) + (p & 1) * dist(p >> 1); }
+};
+template <> struct Codec<3> : PairOrder<3> {};
+template <> struct Codec<5> : PairOrder<5> {};
+template <> struct Codec<6> : PairOrder<6> {};
+
 __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                         uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "

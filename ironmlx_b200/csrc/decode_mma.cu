@@ -219,11 +219,13 @@ void decode_block_order(int bits, int order[16]) {
     if (bits == 4) for (int i = 0; i < 16; ++i) order[i] = Codec<4>::order(i);
     if (bits == 8) for (int i = 0; i < 16; ++i) order[i] = Codec<8>::order(i);
     if (bits == 2) for (int i = 0; i < 16; ++i) order[i] = Codec<2>::order(i);
+    if (bits == 3) for (int i = 0; i < 16; ++i) order[i] = Codec<3>::order(i);
+    if (bits == 5) for (int i = 0; i < 16; ++i) order[i] = Codec<5>::order(i);
+    if (bits == 6) for (int i = 0; i < 16; ++i) order[i] = Codec<6>::order(i);
 }
 
 void expert_block_order(const QFormat& f, int order[16]) {
-    if (f.mode == IMX_MODE_AFFINE && (f.bits == 3 || f.bits == 5 || f.bits == 6)) two_term_block_order(f.bits, order);
-    else decode_block_order(f.mode == IMX_MODE_AFFINE ? f.bits : 0, order);
+    decode_block_order(f.mode == IMX_MODE_AFFINE ? f.bits : 0, order);
 }
 
 bool decode_mma_supported(const ExpertSet& s) {

@@ -72,7 +72,13 @@ int route_slice(int H);                      // K slice of the split-K router (0
 int launch_route(const void* x, int n, int H, const void* Wr, const float* logit_bias, int E, int k,
                  int norm, const void* w_sg, int32_t* topk_idx, float* topk_w, float* shared_gate,
                  void* x16, const int* order16, cudaStream_t stream, float pair_scale_odd = 1.f,
-                 const RouteScratch* rs = nullptr, bool* sums_done = nullptr);
+                 const RouteScratch* rs = nullptr, bool* sums_done = nullptr, int32_t* status = nullptr);
+
+// Router on the tensor cores for larger batches (route_tc.cu); false from `route_tc_supported` leaves the call to the others.
+bool route_tc_supported(const void* x, int n, int H, const void* Wr, int E, const void* x16, const Order16& order);
+int launch_route_tc(const void* x, int n, int H, const void* Wr, const float* logit_bias, int E, int k, int norm, const void* w_sg,
+                    int32_t* topk_idx, float* topk_w, float* shared_gate, void* x16, const Order16& order, int32_t* status,
+                    cudaStream_t stream);
 
 // Order of the 16 values of each block of an fp16 activation row as the
 // expert kernels of a bit width read them (identity for the generic path).
@@ -160,7 +166,6 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
 // The same kernels with the weight as a two-term fp16 sum, for the formats whose weights stay in 32 bits: affine
 // 3/5/6-bit and 4-bit in groups of 32.  kPathTwoTerm is what pick_path answers for them (never a caller's request).
 constexpr int kPathTwoTerm = 100;
-void two_term_block_order(int bits, int order[16]);   // 3, 5, 6 bits (4: the decode kernels' order)
 bool two_term_supported(const ExpertSet& s, bool second_only = false);
 bool two_term_aligned(const ExpertSet& s, bool second_only = false);
 // The current device: its ordinal and SM count (cached per device).
@@ -173,7 +178,7 @@ unsigned long long launch_count();   // kernels this library has launched (or re
 // One-time set-up per (device, kernel family): attributes such as the dynamic shared-memory limit are per
 // device, so a process that drives several GPUs sets them on each.  The first call on a device should come
 // before any stream capture.
-enum { kSetupDecodeTmap = 0, kSetupPrefillTc = 1 };
+enum { kSetupDecodeTmap = 0, kSetupPrefillTc = 1, kSetupRouteTc = 2 };
 bool device_needs_setup(int ordinal, int family);
 void device_mark_setup(int ordinal, int family);
 // Tiled TMA descriptor of a 2-D row-major matrix [rows, cols] of `esize`-byte elements, `ld_bytes` between

@@ -50,18 +50,19 @@
 #include <type_traits>
 
 #include "decode_common.cuh"
+#include "tcgen05.cuh"
 
 namespace imx {
 
 namespace {
 
 using namespace decode;
+using namespace tc;
 
 constexpr int kTileK = 64;
 constexpr int kXBytes = 128 * kTileK * 2;          // activation tile, 16 KB
 constexpr int kWBytes = 128 * kTileK * 2;          // dequantized weight tile (TS = false only), 16 KB
 constexpr int kMaxStages = 8;
-constexpr int kSpin = 1 << 22;
 constexpr uint32_t kTmemCols = 512;                // two 128-column accumulators + the ring of A tiles
 constexpr uint32_t kTmemA = 256;                   // first column of the A ring (32 columns per stage)
 constexpr int kThreadsTc = 640;                    // 20 warps: 4 control, 4 + 4 epilogue, 8 producers
@@ -127,163 +128,6 @@ struct TcParams {
     unsigned long long ord_lut;                    // reduction index at position p of a block of 16, 4 bits each
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Arrival on the barrier at the same offset in CTA 0 of the cluster.  What it announces is in tensor memory (ordered by
-// the tcgen05 fences around it), so that it needs no fence of ordinary memory: with .release.cluster the producers and
-// the epilogue waited for their stores each time, and the first product took 553 instead of 410 us (c3).
-__device__ __forceinline__ void mbar_arrive_cta0(uint32_t bar) {
-    asm volatile(
-        "{\n\t.reg .b32 ra;\n\t"
-        "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
-        "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar)
-        : "memory");
-}
-// One lane of the (converged) warp.  Issued under `lane == 0` a tcgen05.mma cost 94 cycles whatever its N, its operands
-// being moved to uniform registers one lane at a time; under elect.sync 51 (N = 16) to 74 (N = 128), 33 to 64 for a pair.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t e;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
-    return e != 0;
-}
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Bounded wait; false (and the abort flag set) when it gives up or someone else did.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    for (int spin = 0; spin < kSpin; ++spin) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spin & 1023) == 1023 && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    return false;
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y)
-                 : "memory");
-}
-__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// K-major, 128-byte swizzle: rows of 128 bytes, atoms of 8 rows (1024 bytes).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3fffu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// kind::f16 instruction descriptor: D fp32, A/B fp16 K-major, M = m, N = n
-__device__ __forceinline__ uint32_t idesc_for(int m, int n) {
-    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-// D[tmem_d] (+)= A[tmem_a] * B[smem]: A from tensor memory
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
-// The same for a pair of CTAs (issued by CTA 0): M = 256, each CTA's 128 lanes of A and D in its own tensor memory,
-// each CTA's half of B's rows at the same offset of its own shared memory.
-__device__ __forceinline__ void umma_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Arrival on the barrier at this offset in both CTAs once the MMAs issued so far have retired.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"((uint16_t)3)
-                 : "memory");
-}
-__device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// 16 lanes x 64 columns: thread t gets, for each block j of 8 columns, lane t/4 columns 8j + 2(t%4), +1
-// (v[4j], v[4j+1]) and lane t/4 + 8, same columns (v[4j+2], v[4j+3])
-__device__ __forceinline__ void tmem_ld_16x64(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// 32 consecutive columns of this thread's lane <- v
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
-          "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
-          "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-// 16 consecutive columns of this thread's lane <- v; the caller waits with tmem_st_wait
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Four (two) 8 x 8 matrices of 16-bit values in the MMA fragment layout (thread t: row t / 4, columns 2 (t % 4), + 1) to
 // shared memory, transposed: lane 8 m + i names the 16 bytes column i of matrix m goes to.
 __device__ __forceinline__ void stmatrix4_trans(uint32_t addr, uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
@@ -603,21 +447,10 @@ struct Dequant<FMT_NVFP4> {
 // that have no partner at that distance pair with their neighbour.
 template <int BITS>
 struct TwoTerm {
-    static constexpr int D = BITS == 3 ? 6 : (BITS == 6 ? 3 : 4);
+    static constexpr int D = PairOrder<BITS>::D;
     static constexpr int HS = BITS * D - 16;                 // bit of the upper half-word the second code starts at
-    static constexpr int SPAN = BITS == 3 ? 12 : (BITS == 6 ? 6 : 8);   // codes that pair up among themselves
-    // first code of pair p of a block of 16 and the distance of its partner
-    __host__ __device__ static constexpr int first(int p) {
-        const int full = 16 / SPAN * SPAN, rest = p - full / 2;
-        if (rest < 0) return p / D * SPAN + p % D;
-        if (BITS == 6) return rest == 0 ? 12 : 13;           // (12, 15) (13, 14)
-        return full + 2 * rest;
-    }
-    __host__ __device__ static constexpr int dist(int p) {
-        const int full = 16 / SPAN * SPAN, rest = p - full / 2;
-        if (rest < 0) return D;
-        return BITS == 6 && rest == 0 ? 3 : 1;
-    }
+    __host__ __device__ static constexpr int first(int p) { return PairOrder<BITS>::first(p); }
+    __host__ __device__ static constexpr int dist(int p) { return PairOrder<BITS>::dist(p); }
     // the pair as 1024 + q (lower half), 1024 + 2^HS q (upper half)
     template <int BIT, int DIST>
     static __device__ __forceinline__ uint32_t pair(const uint32_t* w) {
@@ -1456,20 +1289,6 @@ bool prefill_tc_supported(const ExpertSet& s, bool second_only) {
     if ((!second_only && !k_ok(s.n_in, f)) || !k_ok(s.n_mid, f)) return false;
     if (s.has_extra && (s.x_mid % 64 || !k_ok(s.x_mid, f))) return false;
     return true;
-}
-
-template <int BITS>
-static void two_term_order(int order[16]) {
-    for (int p = 0; p < 8; ++p) {
-        order[2 * p] = TwoTerm<BITS>::first(p);
-        order[2 * p + 1] = TwoTerm<BITS>::first(p) + TwoTerm<BITS>::dist(p);
-    }
-}
-void two_term_block_order(int bits, int order[16]) {
-    if (bits == 3) two_term_order<3>(order);
-    else if (bits == 5) two_term_order<5>(order);
-    else if (bits == 6) two_term_order<6>(order);
-    else two_term_order<4>(order);
 }
 
 // Do the weight tiles of a unit pair up (64 gate and 64 up rows, 128 output rows a tile)?

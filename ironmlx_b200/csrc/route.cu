@@ -14,7 +14,7 @@
 // plus x; the stage is latency-bound, not bandwidth-bound.
 #include <cooperative_groups.h>
 
-#include "decode_common.cuh"
+#include "route_common.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -22,128 +22,9 @@ namespace imx {
 
 namespace {
 
+using namespace route;
+
 constexpr int kRouteThreads = 256;
-
-// Block order of the fp16 copy by code width (0: rows stay as they are): position p of a block of 16 takes
-// value order16<BITS>(p) of the source block.
-template <int BITS>
-__host__ __device__ constexpr int order16(int p) {
-    if constexpr (BITS == 0) return p;
-    else return decode::Codec<BITS>::order(p);
-}
-// Which of them `order` is, or -1.
-inline int order_bits(const Order16& order) {
-    const int widths[4] = {0, 4, 8, 2};
-    for (int w = 0; w < 4; ++w) {
-        bool same = true;
-        for (int i = 0; i < 16; ++i) {
-            const int want = widths[w] == 0 ? order16<0>(i) : (widths[w] == 4 ? order16<4>(i) : (widths[w] == 8 ? order16<8>(i) : order16<2>(i)));
-            same = same && order.o[i] == want;
-        }
-        if (same) return widths[w];
-    }
-    return -1;
-}
-// One block of 16 bf16 values -> fp16 in block order BITS, pairs 1 and 3 of every 8 stored values times sc_odd:
-// two 16-byte loads, the permutation in registers, two 16-byte stores.
-template <int BITS>
-__device__ __forceinline__ void convert_block16(const __nv_bfloat16* __restrict__ src, __half* __restrict__ dst, float sc_odd) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(src)), b = __ldg(reinterpret_cast<const uint4*>(src) + 1);
-    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    float in[16];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        in[2 * i] = __uint_as_float(w[i] << 16);
-        in[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    }
-    uint32_t o[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const float sc = (q & 1) ? sc_odd : 1.f;
-        const __half2 h = __halves2half2(f32_to_f16_sat(in[order16<BITS>(2 * q)] * sc), f32_to_f16_sat(in[order16<BITS>(2 * q + 1)] * sc));
-        o[q] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-    reinterpret_cast<uint4*>(dst)[0] = make_uint4(o[0], o[1], o[2], o[3]);
-    reinterpret_cast<uint4*>(dst)[1] = make_uint4(o[4], o[5], o[6], o[7]);
-}
-
-
-template <int JMAX>
-__device__ void softmax_topk_warp(const float* s_logits, int E, int k, bool norm, int32_t* out_idx,
-                                  float* out_w) {
-    const int lane = threadIdx.x & 31;
-    float p[JMAX];
-    float m = -INFINITY;
-#pragma unroll
-    for (int j = 0; j < JMAX; ++j) {
-        int e = lane + 32 * j;
-        p[j] = e < E ? s_logits[e] : -INFINITY;
-        m = fmaxf(m, p[j]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    float s = 0.f;
-#pragma unroll
-    for (int j = 0; j < JMAX; ++j) {
-        int e = lane + 32 * j;
-        p[j] = e < E ? expf(p[j] - m) : 0.f;
-        s += p[j];
-    }
-    s = warp_sum(s);
-#pragma unroll
-    for (int j = 0; j < JMAX; ++j) {
-        int e = lane + 32 * j;
-        p[j] = e < E ? p[j] / s : -1.f;   // -1 marks "not selectable"
-    }
-    float my_w = 0.f;
-    int my_i = 0;
-    float wsum = 0.f;
-    // every lane keeps the best of its own candidates (lowest id first among equals); a round is then two
-    // warp reductions (largest probability, lowest id that has it) and a rescan in the winning lane only.
-    // Probabilities are >= 0 and the "taken" mark is -1, so the int view of the floats orders them.
-    float bv;
-    int bj;
-    auto rescan = [&]() {
-        bv = -1.f;
-        bj = 0;
-#pragma unroll
-        for (int j = 0; j < JMAX; ++j) {
-            if (p[j] > bv) {
-                bv = p[j];
-                bj = j;
-            }
-        }
-    };
-    rescan();
-    for (int r = 0; r < k; ++r) {
-        const int mine = __float_as_int(bv);
-        const int top = __reduce_max_sync(0xffffffffu, mine);
-        const int win = __reduce_min_sync(0xffffffffu, mine == top ? lane + 32 * bj : 0x7fffffff);
-        const float wv = __int_as_float(top);
-        if (mine == top && lane + 32 * bj == win) {
-#pragma unroll
-            for (int j = 0; j < JMAX; ++j)
-                if (j == bj) p[j] = -1.f;
-            rescan();
-        }
-        if (lane == (r & 31)) {
-            my_w = wv;
-            my_i = win;
-        }
-        wsum += wv;
-        if ((r & 31) == 31 || r == k - 1) {      // flush up to 32 results
-            int slot = (r & ~31) + lane;
-            if (slot <= r) {
-                out_idx[slot] = my_i;
-                out_w[slot] = my_w;               // normalised below
-            }
-        }
-    }
-    __syncwarp();
-    if (norm) {
-        for (int slot = lane; slot < k; slot += 32) out_w[slot] = out_w[slot] / wsum;
-    }
-}
 
 __global__ void __launch_bounds__(kRouteThreads)
 route_kernel(const __nv_bfloat16* __restrict__ x, int H, const __nv_bfloat16* __restrict__ Wr,
@@ -246,163 +127,12 @@ route_kernel(const __nv_bfloat16* __restrict__ x, int H, const __nv_bfloat16* __
 }
 
 
-// ── prefill-size router: logits on the tensor cores ─────────────────────────
-// 32 tokens x all experts per CTA with mma.sync m16n8k16 (bf16 x bf16 -> fp32):
-// activations and router rows stream through shared memory in K chunks of 64
-// (16-byte cp.async, double buffered), the fp32 logits of the tile land in
-// shared memory and each warp finishes its share of the tokens with the same
-// warp softmax/top-k as the decode-size kernel.  W warps per CTA: each takes
-// E / W experts of the product and 32 / W tokens of the epilogue (eight warps
-// from 64 experts on: the epilogue is half of the kernel's time and serial per
-// warp).
-constexpr int kRT = 32;            // tokens per CTA
-constexpr int kRK = 64;            // K chunk
-constexpr int kRPad = 72;          // bf16 per smem row (64 + 8: conflict-free fragment loads)
-
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-
-template <int NT, int W>   // E = 32 * NT experts, W warps
-__global__ void __launch_bounds__(W * 32)
-route_mma_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, const __nv_bfloat16* __restrict__ Wr,
-                 const float* __restrict__ logit_bias, int k, int norm, const __nv_bfloat16* __restrict__ w_sg,
-                 int32_t* __restrict__ topk_idx, float* __restrict__ topk_w, float* __restrict__ shared_gate,
-                 __half* __restrict__ x16, const Order16 order, const int obits) {
-    constexpr int E = 32 * NT;
-    constexpr int kRThreads = W * 32;
-    constexpr int NW = 4 * NT / W;            // n-tiles of 8 experts per warp
-    static_assert(NW >= 1 && NW * W == 4 * NT, "experts must divide evenly over the warps");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __nv_bfloat16* s_x = reinterpret_cast<__nv_bfloat16*>(smem_raw);                 // [2][kRT][kRPad]
-    __nv_bfloat16* s_w = s_x + 2 * kRT * kRPad;                                      // [2][E][kRPad]
-    float* s_logits = reinterpret_cast<float*>(smem_raw);                            // [kRT][E] (reuses the buffers)
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int tok0 = blockIdx.x * kRT;
-
-    auto load_chunk = [&](int buf, int kc) {
-        // activations: 32 rows x 8 chunks of 16 bytes
-        for (int c = tid; c < kRT * 8; c += kRThreads) {
-            const int r = c >> 3, ch = c & 7;
-            const int tok = tok0 + r;
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_x + (buf * kRT + r) * kRPad + ch * 8);
-            const __nv_bfloat16* src = x + (size_t)(tok < n_tokens ? tok : 0) * H + kc * kRK + ch * 8;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(tok < n_tokens ? 16 : 0) : "memory");
-        }
-        for (int c = tid; c < E * 8; c += kRThreads) {
-            const int r = c >> 3, ch = c & 7;
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_w + (buf * E + r) * kRPad + ch * 8);
-            const __nv_bfloat16* src = Wr + (size_t)r * H + kc * kRK + ch * 8;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, 16;" ::"r"(dst), "l"(src) : "memory");
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-
-    float acc[2][NW][4];
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int n = 0; n < NW; ++n)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.f;
-
-    const int nchunks = H / kRK;
-    load_chunk(0, 0);
-    for (int kc = 0; kc < nchunks; ++kc) {
-        const int buf = kc & 1;
-        if (kc + 1 < nchunks) {
-            load_chunk(buf ^ 1, kc + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        const __nv_bfloat16* xs = s_x + buf * kRT * kRPad;
-        const __nv_bfloat16* ws = s_w + (buf * E + warp * (8 * NW)) * kRPad;
-#pragma unroll
-        for (int kk = 0; kk < kRK / 16; ++kk) {
-            uint32_t af[2][4];
-#pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                const __nv_bfloat16* p = xs + (m * 16 + g) * kRPad + kk * 16 + 2 * t;
-                af[m][0] = *reinterpret_cast<const uint32_t*>(p);
-                af[m][1] = *reinterpret_cast<const uint32_t*>(p + 8 * kRPad);
-                af[m][2] = *reinterpret_cast<const uint32_t*>(p + 8);
-                af[m][3] = *reinterpret_cast<const uint32_t*>(p + 8 * kRPad + 8);
-            }
-#pragma unroll
-            for (int n = 0; n < NW; ++n) {
-                const __nv_bfloat16* p = ws + (n * 8 + g) * kRPad + kk * 16 + 2 * t;
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(p);
-                const uint32_t b1 = *reinterpret_cast<const uint32_t*>(p + 8);
-                mma_bf16(acc[0][n], af[0][0], af[0][1], af[0][2], af[0][3], b0, b1);
-                mma_bf16(acc[1][n], af[1][0], af[1][1], af[1][2], af[1][3], b0, b1);
-            }
-        }
-        __syncthreads();
-    }
-    // logits (+ bias) of the tile into shared memory
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int n = 0; n < NW; ++n) {
-            const int e = warp * (8 * NW) + n * 8 + 2 * t;
-            const float b0 = logit_bias ? logit_bias[e] : 0.f, b1 = logit_bias ? logit_bias[e + 1] : 0.f;
-            s_logits[(m * 16 + g) * E + e] = acc[m][n][0] + b0;
-            s_logits[(m * 16 + g) * E + e + 1] = acc[m][n][1] + b1;
-            s_logits[(m * 16 + g + 8) * E + e] = acc[m][n][2] + b0;
-            s_logits[(m * 16 + g + 8) * E + e + 1] = acc[m][n][3] + b1;
-        }
-    __syncthreads();
-    // each warp finishes its tokens: softmax/top-k, shared gate, fp16 copy
-    for (int r = warp * (kRT / W); r < (warp + 1) * (kRT / W); ++r) {
-        const int tok = tok0 + r;
-        if (tok >= n_tokens) break;
-        softmax_topk_warp<NT>(s_logits + r * E, E, k, norm, topk_idx + (size_t)tok * k, topk_w + (size_t)tok * k);
-        const __nv_bfloat16* xr = x + (size_t)tok * H;
-        if (w_sg != nullptr) {
-            float acc_g = 0.f;
-            for (int c = lane * 8; c < H; c += 256) {
-                const uint4 xv = __ldg(reinterpret_cast<const uint4*>(xr + c));
-                const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w_sg + c));
-                const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&xv);
-                const __nv_bfloat162* wb = reinterpret_cast<const __nv_bfloat162*>(&wv);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 xf = __bfloat1622float2(xb[i]), wf = __bfloat1622float2(wb[i]);
-                    acc_g = fmaf(xf.x, wf.x, acc_g);
-                    acc_g = fmaf(xf.y, wf.y, acc_g);
-                }
-            }
-            acc_g = warp_sum(acc_g);
-            if (lane == 0) shared_gate[tok] = 1.0f / (1.0f + expf(-acc_g));
-        }
-        if (x16 != nullptr && obits >= 0) {
-            // a block of 16 per lane at a time, in the order the expert kernels of this code width read
-            __half* dst = x16 + (size_t)tok * H;
-            for (int c = lane * 16; c < H; c += 32 * 16) {
-                if (obits == 4) convert_block16<4>(xr + c, dst + c, order.pair_scale_odd);
-                else if (obits == 8) convert_block16<8>(xr + c, dst + c, order.pair_scale_odd);
-                else if (obits == 2) convert_block16<2>(xr + c, dst + c, order.pair_scale_odd);
-                else convert_block16<0>(xr + c, dst + c, order.pair_scale_odd);
-            }
-        } else if (x16 != nullptr) {
-            __half2* dst = reinterpret_cast<__half2*>(x16 + (size_t)tok * H);
-            for (int i = lane; i < H / 2; i += 32) {
-                const int blk = (2 * i) & ~15, p = (2 * i) & 15;
-                const float sc = (i & 1) ? order.pair_scale_odd : 1.f;
-                const float a = __bfloat162float(xr[blk + order.o[p]]) * sc;
-                const float b = __bfloat162float(xr[blk + order.o[p + 1]]) * sc;
-                dst[i] = __halves2half2(f32_to_f16_sat(a), f32_to_f16_sat(b));
-            }
-        }
-    }
-}
-
 
 // ── decode-size router on the tensor cores, split over K ────────────────────
 // One CTA per (32 experts, K slice, 32 tokens): the two bf16 tiles are copied to
@@ -577,24 +307,6 @@ route_finish_kernel(int n_tokens, int n_pad, int n_splits, const float* __restri
     }
 }
 
-template <int NT>
-int launch_route_mma(const void* x, int n, int H, const void* Wr, const float* logit_bias, int k, int norm,
-                     const void* w_sg, int32_t* topk_idx, float* topk_w, float* shared_gate, void* x16,
-                     const Order16& order, cudaStream_t stream) {
-    constexpr int E = 32 * NT;
-    const size_t stage = (size_t)2 * (kRT + E) * kRPad * sizeof(__nv_bfloat16);
-    const size_t logits = (size_t)kRT * E * sizeof(float);
-    const size_t smem = stage > logits ? stage : logits;
-    constexpr int W = NT >= 2 ? 8 : 4;
-    IMX_CHECK_CUDA(cudaFuncSetAttribute(route_mma_kernel<NT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    route_mma_kernel<NT, W><<<ceil_div(n, kRT), W * 32, smem, stream>>>(
-        (const __nv_bfloat16*)x, n, H, (const __nv_bfloat16*)Wr, logit_bias, k, norm, (const __nv_bfloat16*)w_sg,
-        topk_idx, topk_w, shared_gate, (__half*)x16, order,
-        ((uintptr_t)x % 16 == 0 && (uintptr_t)x16 % 16 == 0) ? order_bits(order) : -1); IMX_LAUNCHED();
-    IMX_CHECK_CUDA(cudaGetLastError());
-    return IMX_OK;
-}
-
 }  // namespace
 
 int route_slice(int H) {
@@ -607,7 +319,7 @@ int route_slice(int H) {
 int launch_route(const void* x, int n, int H, const void* Wr, const float* logit_bias, int E, int k,
                  int norm, const void* w_sg, int32_t* topk_idx, float* topk_w, float* shared_gate,
                  void* x16, const int* order16, cudaStream_t stream, float pair_scale_odd, const RouteScratch* rs,
-                 bool* sums_done) {
+                 bool* sums_done, int32_t* status) {
     IMX_REQUIRE(n >= 0 && H > 0 && H % 16 == 0, "route: hidden (%d) must be a positive multiple of 16", H);
     Order16 order;
     for (int i = 0; i < 16; ++i) order.o[i] = (int8_t)(order16 ? order16[i] : i);
@@ -631,15 +343,8 @@ int launch_route(const void* x, int n, int H, const void* Wr, const float* logit
         if (sums_done != nullptr) *sums_done = rs->gsum_x != nullptr;
         return IMX_OK;
     }
-    if (n >= 256 && H % kRK == 0 && E % 32 == 0 && E <= 256) {
-        switch (E / 32) {
-            case 1: return launch_route_mma<1>(x, n, H, Wr, logit_bias, k, norm, w_sg, topk_idx, topk_w, shared_gate, x16, order, stream);
-            case 2: return launch_route_mma<2>(x, n, H, Wr, logit_bias, k, norm, w_sg, topk_idx, topk_w, shared_gate, x16, order, stream);
-            case 4: return launch_route_mma<4>(x, n, H, Wr, logit_bias, k, norm, w_sg, topk_idx, topk_w, shared_gate, x16, order, stream);
-            case 8: return launch_route_mma<8>(x, n, H, Wr, logit_bias, k, norm, w_sg, topk_idx, topk_w, shared_gate, x16, order, stream);
-            default: break;
-        }
-    }
+    if (route_tc_supported(x, n, H, Wr, E, x16, order))
+        return launch_route_tc(x, n, H, Wr, logit_bias, E, k, norm, w_sg, topk_idx, topk_w, shared_gate, x16, order, status, stream);
     // cluster size: enough CTAs to cover the GPU at small N, experts split evenly
     int cs = 1;
     while (cs < 8 && (long)n * cs < 296 && E / (cs * 2) >= 16) cs *= 2;
