@@ -342,7 +342,21 @@ static int forward_impl(const imx_moe_config* cfg, const imx_moe_weights* w, con
     path_block_order(path, f, order);
     auto mark = [&](int i) -> cudaError_t { return ev ? cudaEventRecord(ev[i], stream) : cudaSuccess; };
     const bool tmap_decode = path == IMX_PATH_DECODE && decode_tmap_supported(set);
-    RouteScratch rscratch = {ws.route_partials, ws.route_sg, tmap_decode ? ws.gsum_x : nullptr, nullptr, nullptr};
+    SortExtras ex;
+    ex.topk_w = ws.topk_w;
+    ex.top_k = c.top_k;
+    ex.tok_of_slot = ws.tok_of_slot;
+    ex.w_of_slot = ws.w_of_slot;
+    ex.shared_gate = has_shared ? ws.shared_gate : nullptr;
+    ex.n_tokens = n_tokens;
+    ex.units = ws.units;
+    ex.n_units = ws.n_units;
+    ex.unit_rows = unit_rows_for(path);
+    ex.sched = ws.sw.sched;
+    ex.sched_ints = ws.sw.n_ints;
+    const RouteSort rsort = {ex, ws.counts, ws.offsets, ws.perm, ws.inv_perm, ws.status + kStatusRouteArrivals};
+    RouteScratch rscratch = {ws.route_partials, ws.route_sg, tmap_decode ? ws.gsum_x : nullptr, nullptr, nullptr, &rsort};
+    bool sort_done = false;
     bool sums_done = false;
     IMX_CHECK_CUDA(mark(0));
     const void* router_in = x;
@@ -362,22 +376,11 @@ static int forward_impl(const imx_moe_config* cfg, const imx_moe_weights* w, con
     IMX_TRY(launch_route(router_in, n_tokens, c.hidden, w->router_w, w->router_logit_bias, c.num_experts, c.top_k,
                          c.norm_topk_prob, has_shared ? w->shared_expert_gate_w : nullptr, ws.topk_idx,
                          ws.topk_w, ws.shared_gate, ws.x16, order, stream,
-                         tmap_decode ? 0.0625f : 1.f, ws.route_partials ? &rscratch : nullptr, &sums_done, ws.status));
+                         tmap_decode ? 0.0625f : 1.f, ws.route_partials ? &rscratch : nullptr, &sums_done, ws.status, &sort_done));
     IMX_CHECK_CUDA(mark(1));
-    SortExtras ex;
-    ex.topk_w = ws.topk_w;
-    ex.top_k = c.top_k;
-    ex.tok_of_slot = ws.tok_of_slot;
-    ex.w_of_slot = ws.w_of_slot;
-    ex.shared_gate = has_shared ? ws.shared_gate : nullptr;
-    ex.n_tokens = n_tokens;
-    ex.units = ws.units;
-    ex.n_units = ws.n_units;
-    ex.unit_rows = unit_rows_for(path);
-    ex.sched = ws.sw.sched;
-    ex.sched_ints = ws.sw.n_ints;
-    IMX_TRY(launch_sort(ws.topk_idx, A, c.num_experts, ws.counts, ws.offsets, ws.perm, ws.inv_perm,
-                        ws.sort_scratch, ws.sort_scratch_bytes, &ex, stream));
+    if (!sort_done)
+        IMX_TRY(launch_sort(ws.topk_idx, A, c.num_experts, ws.counts, ws.offsets, ws.perm, ws.inv_perm,
+                            ws.sort_scratch, ws.sort_scratch_bytes, &ex, stream));
     IMX_CHECK_CUDA(mark(2));
     GroupedArgs ga = {};
     ga.set = set;
@@ -547,7 +550,7 @@ int imx_moe_route_ws(const void* x, int n_tokens, int hidden, const void* router
     RouteWs ws = carve_route(n_tokens, hidden, num_experts, scratch);
     IMX_REQUIRE(ws.bytes == 0 || (scratch != nullptr && ((uintptr_t)scratch % 256) == 0 && scratch_bytes >= ws.bytes),
                 "route: scratch of %zu bytes (256-byte aligned) needed, %zu given", ws.bytes, scratch_bytes);
-    RouteScratch rs = {ws.partials, ws.sg, nullptr, nullptr, nullptr};
+    RouteScratch rs = {ws.partials, ws.sg, nullptr, nullptr, nullptr, nullptr};
     return launch_route(x, n_tokens, hidden, router_w, logit_bias, num_experts, top_k, norm_topk_prob,
                         shared_gate_w, topk_idx, topk_w, shared_gate, x_f16, nullptr, (cudaStream_t)stream, 1.f,
                         ws.partials ? &rs : nullptr, nullptr);

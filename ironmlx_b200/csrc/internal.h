@@ -65,6 +65,16 @@ struct RouteScratch {
     float* gsum_x;        // [n][H / 64] group sums of the fp16 copy in units of 2^-24, or nullptr
     const float* inv_rms; // [n] per-token RMSNorm factor: the tiles of x are normalised as they are loaded (or nullptr)
     const void* ln_weight;// bf16 [H] RMSNorm weight that goes with inv_rms (or nullptr)
+    const struct RouteSort* sort;   // the dispatch sort is wanted in the router's last launch (or nullptr)
+};
+// Outputs of the dispatch sort done by the router: the CTA that finishes last sorts all assignments.
+struct RouteSort {
+    SortExtras extras;
+    int32_t* counts;
+    int32_t* offsets;
+    int32_t* perm;
+    int32_t* inv_perm;
+    int32_t* arrivals;    // one zeroed word, left zero
 };
 constexpr int kRouteSplitMaxTokens = 1024;   // the split-K router serves batches below this
 int route_slice(int H);                      // K slice of the split-K router (0: not applicable)
@@ -72,7 +82,8 @@ int route_slice(int H);                      // K slice of the split-K router (0
 int launch_route(const void* x, int n, int H, const void* Wr, const float* logit_bias, int E, int k,
                  int norm, const void* w_sg, int32_t* topk_idx, float* topk_w, float* shared_gate,
                  void* x16, const int* order16, cudaStream_t stream, float pair_scale_odd = 1.f,
-                 const RouteScratch* rs = nullptr, bool* sums_done = nullptr, int32_t* status = nullptr);
+                 const RouteScratch* rs = nullptr, bool* sums_done = nullptr, int32_t* status = nullptr,
+                 bool* sort_done = nullptr);
 
 // Router on the tensor cores for larger batches (route_tc.cu); false from `route_tc_supported` leaves the call to the others.
 bool route_tc_supported(const void* x, int n, int H, const void* Wr, int E, const void* x16, const Order16& order);

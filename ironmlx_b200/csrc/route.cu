@@ -14,7 +14,10 @@
 // plus x; the stage is latency-bound, not bandwidth-bound.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "route_common.cuh"
+#include "sort_small.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -261,15 +264,27 @@ route_splitk_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, co
 
 // Second half of the split-K router: one warp per token adds the K slices in slice
 // order (so the sums do not depend on timing) and does softmax / top-k.
-__global__ void __launch_bounds__(kSkThreads)
+// SORT: the CTA that gets here last sorts the assignments of all of them, every CTA clears its share of the scheduler
+// words.  For the smallest batches, where a launch of its own costs more than it sorts (a call of 1 token 52.5 -> 51.0 us,
+// of 19 tokens 95.1 -> 93.1); at 64 tokens the sixteen tokens a CTA of 512 threads finishes take longer than the launch
+// saved (119.4 -> 120.1 us as a graph), so that more than kRouteSortTokens keep four tokens a CTA and the sort's launch.
+constexpr int kFinThreadsSort = 512;
+constexpr int kRouteSortTokens = 32;
+
+template <bool SORT>
+__global__ void __launch_bounds__(SORT ? kFinThreadsSort : kSkThreads)
 route_finish_kernel(int n_tokens, int n_pad, int n_splits, const float* __restrict__ logit_bias, int E, int k, int norm,
-                    int has_sg, int32_t* __restrict__ topk_idx, float* __restrict__ topk_w,
-                    float* __restrict__ shared_gate, const RouteScratch rs) {
+                    int has_sg, int32_t* topk_idx, float* topk_w, float* shared_gate, const RouteScratch rs, const SortAux aux,
+                    int32_t* __restrict__ counts, int32_t* __restrict__ offsets, int32_t* __restrict__ perm,
+                    int32_t* __restrict__ inv_perm, int32_t* __restrict__ arrivals) {
+    constexpr int kFinThreads = SORT ? kFinThreadsSort : kSkThreads;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* my_logits = reinterpret_cast<float*>(smem_raw) + warp * E;
-    const int tok = blockIdx.x * (kSkThreads / 32) + warp;
-    if (tok >= n_tokens) return;
+    const int tok = blockIdx.x * (kFinThreads / 32) + warp;
+    if (SORT)
+        for (int i = blockIdx.x * kFinThreads + threadIdx.x; i < aux.sched_ints; i += gridDim.x * kFinThreads) aux.sched[i] = 0;
+    if (tok < n_tokens) {
     // 4 experts per lane and pass (16-byte loads), all slices of a pass in flight together
     for (int e = lane * 4; e < E; e += 128) {
         const float* p = rs.partials + (size_t)tok * E + e;
@@ -305,6 +320,20 @@ route_finish_kernel(int n_tokens, int n_pad, int n_splits, const float* __restri
         for (int s = 0; s < n_splits; ++s) v += __ldcg(rs.sg_partials + (size_t)s * n_pad + tok);
         shared_gate[tok] = 1.0f / (1.0f + expf(-v));
     }
+    }
+    if (SORT) {
+        __shared__ int s_last;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(arrivals, 1) == (int)gridDim.x - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        if (threadIdx.x == 0) *arrivals = 0;
+        SortAux rest = aux;
+        rest.sched = nullptr;
+        sort_small_block<kFinThreads>(topk_idx, n_tokens * k, E, counts, offsets, perm, inv_perm, rest, reinterpret_cast<int*>(smem_raw));
+    }
 }
 
 }  // namespace
@@ -319,7 +348,7 @@ int route_slice(int H) {
 int launch_route(const void* x, int n, int H, const void* Wr, const float* logit_bias, int E, int k,
                  int norm, const void* w_sg, int32_t* topk_idx, float* topk_w, float* shared_gate,
                  void* x16, const int* order16, cudaStream_t stream, float pair_scale_odd, const RouteScratch* rs,
-                 bool* sums_done, int32_t* status) {
+                 bool* sums_done, int32_t* status, bool* sort_done) {
     IMX_REQUIRE(n >= 0 && H > 0 && H % 16 == 0, "route: hidden (%d) must be a positive multiple of 16", H);
     Order16 order;
     for (int i = 0; i < 16; ++i) order.o[i] = (int8_t)(order16 ? order16[i] : i);
@@ -328,6 +357,7 @@ int launch_route(const void* x, int n, int H, const void* Wr, const float* logit
     IMX_REQUIRE(k >= 1 && k <= E, "route: top_k (%d) must be in 1..num_experts (%d)", k, E);
     IMX_REQUIRE(w_sg == nullptr || shared_gate != nullptr, "route: shared gate weight without output");
     if (sums_done != nullptr) *sums_done = false;
+    if (sort_done != nullptr) *sort_done = false;
     if (n == 0) return IMX_OK;
     const int ks = route_slice(H);
     if (rs != nullptr && rs->partials != nullptr && n < kRouteSplitMaxTokens && ks > 0 && E % 32 == 0 && x16 != nullptr) {
@@ -337,8 +367,20 @@ int launch_route(const void* x, int n, int H, const void* Wr, const float* logit
             (const __nv_bfloat16*)x, n, H, (const __nv_bfloat16*)Wr, logit_bias, E, k, norm, (const __nv_bfloat16*)w_sg,
             topk_idx, topk_w, shared_gate, (__half*)x16, order, ks, *rs); IMX_LAUNCHED();
         IMX_CHECK_CUDA(cudaGetLastError());
-        route_finish_kernel<<<ceil_div(n, kSkThreads / 32), kSkThreads, (size_t)(kSkThreads / 32) * E * sizeof(float), stream>>>(
-            n, (int)grid.z * 32, (int)grid.y, logit_bias, E, k, norm, w_sg != nullptr, topk_idx, topk_w, shared_gate, *rs); IMX_LAUNCHED();
+        const bool sorts = rs->sort != nullptr && sort_done != nullptr && n <= kRouteSortTokens && E <= kSmallSortExperts &&
+                           n * k <= kSmallSortIters * kFinThreadsSort;
+        if (sorts) {
+            const RouteSort& so = *rs->sort;
+            const size_t ints = std::max((size_t)(kFinThreadsSort / 32) * E, small_sort_ints(kFinThreadsSort / 32, E));
+            route_finish_kernel<true><<<ceil_div(n, kFinThreadsSort / 32), kFinThreadsSort, ints * sizeof(int), stream>>>(
+                n, (int)grid.z * 32, (int)grid.y, logit_bias, E, k, norm, w_sg != nullptr, topk_idx, topk_w, shared_gate, *rs,
+                make_sort_aux(&so.extras), so.counts, so.offsets, so.perm, so.inv_perm, so.arrivals); IMX_LAUNCHED();
+            *sort_done = true;
+        } else {
+            route_finish_kernel<false><<<ceil_div(n, kSkThreads / 32), kSkThreads, (size_t)(kSkThreads / 32) * E * sizeof(float), stream>>>(
+                n, (int)grid.z * 32, (int)grid.y, logit_bias, E, k, norm, w_sg != nullptr, topk_idx, topk_w, shared_gate, *rs,
+                SortAux{}, nullptr, nullptr, nullptr, nullptr, nullptr); IMX_LAUNCHED();
+        }
         IMX_CHECK_CUDA(cudaGetLastError());
         if (sums_done != nullptr) *sums_done = rs->gsum_x != nullptr;
         return IMX_OK;
