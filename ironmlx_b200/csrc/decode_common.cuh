@@ -234,7 +234,9 @@ __device__ __forceinline__ void epilogue(const GroupedArgs& a, const TaskCtx& c,
                     if (slot_l < c.rows) {
                         const int slot = c.slot0 + slot_l;
                         const float sc = a.row_scale ? a.row_scale[slot] : 1.f;
-                        a.out[(size_t)slot * a.set.n_in + row] = acc[T][i] * c.gs[T] * sc;
+                        const float v = acc[T][i] * c.gs[T] * sc;
+                        if (a.out_bf16 != nullptr) a.out_bf16[(size_t)slot * a.set.n_in + row] = __float2bfloat16_rn(v);
+                        else a.out[(size_t)slot * a.set.n_in + row] = v;
                     }
                 }
         }

@@ -281,7 +281,8 @@ __device__ __forceinline__ void finish(const GroupedArgs& a, const FpTask& c, fl
                     if (slot_l < c.rows) {
                         const int slot = c.slot0 + slot_l;
                         const float sc = a.row_scale ? a.row_scale[slot] : 1.f;
-                        a.out[(size_t)slot * a.set.n_in + row] = r[T][i] * sc;
+                        if (a.out_bf16 != nullptr) a.out_bf16[(size_t)slot * a.set.n_in + row] = __float2bfloat16_rn(r[T][i] * sc);
+                        else a.out[(size_t)slot * a.set.n_in + row] = r[T][i] * sc;
                     }
                 }
         }

@@ -821,7 +821,11 @@ decode_second_kernel(const GroupedArgs a, const DecodeParams p, const __grid_con
                     const int slot_l = 2 * t + sl;
                     const int row = c_pair * 32 + T * 16 + 2 * g;
                     const float sc = kUnscale * (sl ? c_rs1 : c_rs0);
-                    if (slot_l < c_unit.rows)
+                    if (slot_l >= c_unit.rows) continue;
+                    if (a.out_bf16 != nullptr)
+                        *reinterpret_cast<__nv_bfloat162*>(a.out_bf16 + (size_t)(c_unit.slot0 + slot_l) * S.n_in + row) =
+                            __floats2bfloat162_rn(acc[T][sl] * sc, acc[T][2 + sl] * sc);
+                    else
                         *reinterpret_cast<float2*>(a.out + (size_t)(c_unit.slot0 + slot_l) * S.n_in + row) =
                             make_float2(acc[T][sl] * sc, acc[T][2 + sl] * sc);
                 }

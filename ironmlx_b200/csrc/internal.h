@@ -150,6 +150,7 @@ struct GroupedArgs {
     const float* row_scale;        // per slot or nullptr
     float* out;                    // fp32 [n_slots, n_in]
     __half* out16;                 // prefill path only: the same rows as fp16 instead (out is then unused), or nullptr
+    __nv_bfloat16* out_bf16;       // second product alone: the rows rounded to bf16 instead (out, out16 are then unused), or nullptr
     const int32_t* out_index;      // prefill path only: output row of each slot (nullptr: the slot itself)
     int32_t* status;               // device status word
     int second_only;               // run the second product alone: out = act . down^T (a plain quantized matmul)

@@ -166,6 +166,11 @@ __device__ __forceinline__ uint32_t pack_f16_sat(float lo, float hi) {
     asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
     return d;
 }
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
 // silu with the approximate exponential and reciprocal (relative error ~1e-6, far inside the fp16 rounding that follows)
 __device__ __forceinline__ float silu_fast(float g) {
     float e, r;
@@ -738,7 +743,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             // [lane group of 16][gate, up], or the weight rows 16 gs + 8 r8 + lane / 4 of the warp's 32; second product
             // with one weight row a lane (fp32 rows): [0]
             float rf[4] = {1.f, 1.f, 1.f, 1.f};
-            const bool frag_rows = !SWIGLU && WIDE && a.row_scale == nullptr && a.out16 != nullptr;
+            const bool frag_rows = !SWIGLU && WIDE && a.row_scale == nullptr && (a.out16 != nullptr || a.out_bf16 != nullptr);
             if (SWIGLU) {
 #pragma unroll
                 for (int gs = 0; gs < 2; ++gs) {
@@ -866,8 +871,12 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                                 for (int r8 = 0; r8 < 2; ++r8) {
                                     float x0 = __uint_as_float(v[4 * j + 2 * r8]), x1 = __uint_as_float(v[4 * j + 2 * r8 + 1]);
                                     if (!AFFINE || TWO) { x0 *= rf[2 * gs + r8]; x1 *= rf[2 * gs + r8]; }
-                                    peak = fmaxf(peak, fmaxf(8 * j < n_ok ? fabsf(x0) : 0.f, 8 * j + 1 < n_ok ? fabsf(x1) : 0.f));
-                                    h[2 * gs + r8][j] = pack_f16_sat(x0, x1);
+                                    if (a.out_bf16 != nullptr) {
+                                        h[2 * gs + r8][j] = pack_bf16(x0, x1);
+                                    } else {
+                                        peak = fmaxf(peak, fmaxf(8 * j < n_ok ? fabsf(x0) : 0.f, 8 * j + 1 < n_ok ? fabsf(x1) : 0.f));
+                                        h[2 * gs + r8][j] = pack_f16_sat(x0, x1);
+                                    }
                                 }
                         }
                     };
@@ -878,6 +887,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                         __syncwarp();
                     };
                     auto flush = [&](int c) {
+                        uint16_t* rows16 = a.out_bf16 != nullptr ? reinterpret_cast<uint16_t*>(a.out_bf16) : reinterpret_cast<uint16_t*>(a.out16);
                         const int sl0 = (eh * 2 + c) * 64;
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
@@ -886,7 +896,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                             if (sl0 + sl < t.rows) {
                                 const int slot = t.slot0 + sl0 + sl;
                                 const int orow = a.out_index != nullptr ? a.out_index[slot] : slot;
-                                st_global_128(a.out16 + (size_t)orow * a.set.n_in + t.ntile * 128 + q * 32 + (lane & 3) * 8, v);
+                                st_global_128(rows16 + (size_t)orow * a.set.n_in + t.ntile * 128 + q * 32 + (lane & 3) * 8, v);
                             }
                         }
                         __syncwarp();
@@ -938,6 +948,13 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                             const int r0 = __shfl_sync(0xffffffffu, orow, i), r1 = __shfl_sync(0xffffffffu, orow, i + 1);
                             if (i < n_ok) st_global_u16(a.out16 + (size_t)r0 * a.set.n_in + col, h);
                             if (i + 1 < n_ok) st_global_u16(a.out16 + (size_t)r1 * a.set.n_in + col, h >> 16);
+                        }
+                    } else if (a.out_bf16 != nullptr) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 2) {
+                            const uint32_t h = pack_bf16(o[i], o[i + 1]);
+                            if (i < n_ok) st_global_u16(a.out_bf16 + o0 + (size_t)i * a.set.n_in, h);
+                            if (i + 1 < n_ok) st_global_u16(a.out_bf16 + o0 + (size_t)(i + 1) * a.set.n_in, h >> 16);
                         }
                     } else if (a.out16 != nullptr) {
 #pragma unroll
@@ -1352,7 +1369,7 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
         return make_plan(f, fmt, K_max, K_min, wide, xr, ts, out);
     };
     Plan gu = {}, dn = {};
-    const int epi_second = a.out16 != nullptr ? kEpiSecond : 0;
+    const int epi_second = a.out16 != nullptr || a.out_bf16 != nullptr ? kEpiSecond : 0;
     if (variant == 3) {
         IMX_REQUIRE((a.second_only || wide_plan(f, fmt, s.n_in, s.n_in, first_even(s), kEpiFirst, &gu)) &&
                         wide_plan(f, fmt, mid_max, mid_min, second_even(s), epi_second, &dn),
