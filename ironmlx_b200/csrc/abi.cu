@@ -176,10 +176,24 @@ int make_expert_set(const imx_moe_config& c, const QFormat& f, const imx_qtensor
 bool is_prefill(int path) {
     return path == IMX_PATH_PREFILL || path == IMX_PATH_PREFILL_SMEM || path == IMX_PATH_PREFILL_PLAIN;
 }
-int unit_rows_for(int path) { return is_prefill(path) || path == kPathTwoTerm ? kPrefillUnitRows : kUnitRows; }
+int unit_rows_for(int path) { return is_prefill(path) || path == kPathTwoTerm || path == kPathTcRows32 ? kPrefillUnitRows : kUnitRows; }
 bool is_decode(int path) { return path == IMX_PATH_DECODE || path == IMX_PATH_DECODE_REGS; }
 bool decode_supported(const ExpertSet& s) { return decode_mma_supported(s) || decode_fp_supported(s); }
 
+// Between decode and prefill sizes the decode kernels take an expert's rows through its weights eight at a time, the
+// tensor-core kernels 256 at a time; both keep rows in fp32 and weights exact (block-scaled floats) or in 32 bits
+// (two-term).  Rows an expert (on average) from which the latter are faster, measured on a B200 as us a block:
+//   mxfp8  8   (256 experts of 2048 x 512: 4 rows 310 / 310, 8 rows 425 / 320, 28 rows 1093 / 362; 64 of 1024 x 512: 4 rows 77 / 89)
+//   nvfp4  16  (8 rows 239 / 306, 16 rows 384 / 319, 28 rows 591 / 343)
+static long rows32_from(const ExpertSet& s) { return (s.fmt.mode == IMX_MODE_MXFP8 ? 8L : 16L) * s.num_experts; }
+//   affine, register-pipelined decode kernel  16  (8-bit: 8 rows 400 / 509, 16 rows 671 / 519, 28 rows 1080 / 557; 2-bit:
+//          16 rows 546 / 468), and 128 where the weight tiles do not fill the GPU (16 experts of 512 x 256: 64 rows
+//          62.5 / 70.4, 128 rows 76.8 / 72.7, 256 rows 112 / 79)
+//   affine 4-bit in groups of 64, tensor-map decode kernel: not below prefill sizes (28 rows 486 / 546)
+static long two_term_from(const ExpertSet& s) {
+    if (decode_tmap_supported(s)) return 1L << 40;
+    return ((long)s.num_experts * s.n_mid / 128 >= 148 ? 16L : 128L) * s.num_experts;
+}
 // Which expert kernels run for this call.  AUTO: tensor-memory GEMM tiles once
 // experts see enough rows to fill them, the decode kernels below that.
 int pick_path(const imx_moe_config& c, const ExpertSet& s, long n_rows, int* path) {
@@ -187,8 +201,9 @@ int pick_path(const imx_moe_config& c, const ExpertSet& s, long n_rows, int* pat
     const bool many = n_rows >= 32L * s.num_experts;
     if (p == IMX_PATH_AUTO) {
         if (many && prefill_tc_supported(s)) p = IMX_PATH_PREFILL;
-        else if (decode_supported(s)) p = IMX_PATH_DECODE;
-        else p = two_term_supported(s) && two_term_aligned(s) ? kPathTwoTerm : IMX_PATH_GENERIC;
+        else if (n_rows >= rows32_from(s) && tc_rows32_supported(s) && tc_aligned(s)) p = kPathTcRows32;
+        else if (decode_supported(s) && !(n_rows >= two_term_from(s) && two_term_supported(s) && tc_aligned(s))) p = IMX_PATH_DECODE;
+        else p = two_term_supported(s) && tc_aligned(s) ? kPathTwoTerm : IMX_PATH_GENERIC;
     }
     IMX_REQUIRE(!(p == IMX_PATH_PREFILL || p == IMX_PATH_PREFILL_SMEM || p == IMX_PATH_PREFILL_PLAIN) || prefill_tc_supported(s),
                 "the prefill path supports affine 2/4/8-bit, mxfp8 and nvfp4 with hidden %% 128 == 0, intermediate %% 64 == 0 "
@@ -211,6 +226,7 @@ int run_experts(int path, const GroupedArgs& ga, cudaStream_t stream, cudaEvent_
     if (path == IMX_PATH_PREFILL_PLAIN) return launch_prefill_tc(ga, stream, mid, 1);
     if (path == IMX_PATH_PREFILL_SMEM) return launch_prefill_tc(ga, stream, mid, 2);
     if (path == kPathTwoTerm) return launch_prefill_tc(ga, stream, mid, 3);
+    if (path == kPathTcRows32) return launch_prefill_tc(ga, stream, mid, 0);
     if (is_decode(path) && decode_fp_supported(ga.set)) return launch_decode_fp(ga, stream, mid);
     if (path == IMX_PATH_DECODE && decode_tmap_supported(ga.set)) return launch_decode_tmap(ga, stream, mid);
     if (is_decode(path)) return launch_decode_mma(ga, stream, mid);

@@ -79,8 +79,8 @@ struct Codec<2> {
 // their neighbour (6-bit: (12, 15) and (13, 14)).
 template <int BITS>
 struct PairOrder {
-    static constexpr int D = BITS == 3 ? 6 : (BITS == 6 ? 3 : 4);
-    static constexpr int SPAN = BITS == 3 ? 12 : (BITS == 6 ? 6 : 8);   // codes that pair up among themselves
+    static constexpr int D = BITS == 2 ? 8 : (BITS == 3 ? 6 : (BITS == 6 ? 3 : (BITS == 8 ? 2 : 4)));
+    static constexpr int SPAN = BITS == 3 ? 12 : 2 * D;      // codes that pair up among themselves
     // first code of pair p of a block of 16 and the distance of its partner
     __host__ __device__ static constexpr int first(int p) {
         const int full = 16 / SPAN * SPAN, rest = p - full / 2;

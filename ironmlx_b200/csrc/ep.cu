@@ -391,7 +391,8 @@ int forward_gathered(imx_ep_ctx& x, const imx_moe_weights* w, const void* xin, i
         cd.path = IMX_PATH_DECODE;
         if (pick_path(cd, set, (long)A / R, &path) != IMX_OK) path = IMX_PATH_GENERIC;
     }
-    if (path == kPathTwoTerm) path = IMX_PATH_GENERIC;   // (the workspace of this schedule is not laid out for it)
+    // (the workspace of this schedule is not laid out for the fp32-row tensor-core paths)
+    if (path == kPathTcRows32 || path == kPathTwoTerm) path = decode_supported(set) ? IMX_PATH_DECODE : IMX_PATH_GENERIC;
     const bool tc = is_prefill(path);                // tensor-core kernels: fp16 rows, routing weight applied in the combine
     const bool tmap_decode = path == IMX_PATH_DECODE && decode_tmap_supported(set);
 

@@ -178,8 +178,11 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
 // The same kernels with the weight as a two-term fp16 sum, for the formats whose weights stay in 32 bits: affine
 // 3/5/6-bit and 4-bit in groups of 32.  kPathTwoTerm is what pick_path answers for them (never a caller's request).
 constexpr int kPathTwoTerm = 100;
+// The tensor-core kernels with fp32 expert rows, for batches whose rows the decode kernels keep in fp32 (mxfp8, nvfp4).
+constexpr int kPathTcRows32 = 101;
 bool two_term_supported(const ExpertSet& s, bool second_only = false);
-bool two_term_aligned(const ExpertSet& s, bool second_only = false);
+bool tc_aligned(const ExpertSet& s, bool second_only = false);
+bool tc_rows32_supported(const ExpertSet& s);
 // The current device: its ordinal and SM count (cached per device).
 struct DeviceInfo {
     int ordinal;
@@ -272,6 +275,7 @@ int pick_path(const imx_moe_config& c, const ExpertSet& s, long n_rows, int* pat
 void path_block_order(int path, const QFormat& f, int order[16]);
 int run_experts(int path, const GroupedArgs& ga, cudaStream_t stream, cudaEvent_t mid = nullptr);
 bool is_prefill(int path);
+bool decode_supported(const ExpertSet& s);
 int unit_rows_for(int path);
 int max_units_for(int A, int E, int n_shared_tokens);
 

@@ -68,14 +68,14 @@ constexpr uint32_t kTmemA = 256;                   // first column of the A ring
 constexpr int kThreadsTc = 640;                    // 20 warps: 4 control, 4 + 4 epilogue, 8 producers
 
 // FMT_T*: affine weights as a two-term fp16 sum (hi + lo), see TwoTerm below.
-enum { FMT_A4 = 0, FMT_A8 = 1, FMT_A2 = 2, FMT_MXFP8 = 3, FMT_NVFP4 = 4, FMT_T3 = 5, FMT_T4 = 6, FMT_T5 = 7, FMT_T6 = 8 };
-__host__ __device__ constexpr bool two_term(int fmt) { return fmt >= FMT_T3; }
-__host__ __device__ constexpr int two_term_bits(int fmt) { return fmt - FMT_T3 + 3; }
+enum { FMT_A4 = 0, FMT_A8 = 1, FMT_A2 = 2, FMT_MXFP8 = 3, FMT_NVFP4 = 4, FMT_T2 = 5, FMT_T3 = 6, FMT_T4 = 7, FMT_T5 = 8, FMT_T6 = 9, FMT_T8 = 10 };
+__host__ __device__ constexpr bool two_term(int fmt) { return fmt >= FMT_T2; }
+__host__ __device__ constexpr int two_term_bits(int fmt) { return fmt == FMT_T8 ? 8 : fmt - FMT_T2 + 2; }
 // Bytes of one row the copy engine brings per K step of 64 values.  3- and 5-bit rows advance by 24 and 40 bytes a
 // step and a copy starts on a multiple of 16: the box starts at the multiple below and is wide enough for both
 // positions.  48-byte rows spread eight lanes' 16-byte loads over all banks without a swizzle.
 __host__ __device__ constexpr int q_row_bytes(int fmt) {
-    return fmt == FMT_A8 || fmt == FMT_MXFP8 ? 64 : (fmt == FMT_A2 ? 16 : (fmt == FMT_T3 || fmt == FMT_T5 || fmt == FMT_T6 ? 48 : 32));
+    return fmt == FMT_A8 || fmt == FMT_MXFP8 || fmt == FMT_T8 ? 64 : (fmt == FMT_A2 || fmt == FMT_T2 ? 16 : (fmt == FMT_T3 || fmt == FMT_T5 || fmt == FMT_T6 ? 48 : 32));
 }
 // First byte of K step ks's box in a packed row (a multiple of 16).
 __host__ __device__ constexpr int q_step_byte(int fmt, int ks) {
@@ -114,7 +114,7 @@ struct Bars {                                      // shared-memory control bloc
 
 struct TcMaps {
     CUtensorMap x;                                 // slot-ordered activations
-    CUtensorMap w[3], s[3], b[3];                  // [0] stacked routed matrix, [1]/[2] the extra expert's
+    CUtensorMap w[3];                              // packed codes: [0] stacked routed matrix, [1]/[2] the extra expert's
 };
 
 struct TcParams {
@@ -139,6 +139,12 @@ __device__ __forceinline__ void stmatrix2_trans(uint32_t addr, uint32_t m0, uint
 }
 __device__ __forceinline__ void st_global_128(void* p, uint4 v) {
     asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+// `bytes` consecutive bytes (16-byte aligned, a multiple of 16) to shared memory.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
 }
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     uint2 v;
@@ -496,12 +502,30 @@ struct TwoTerm {
 __device__ __forceinline__ float pow2_f32(int e) {           // e in [-126, 127]
     return __uint_as_float((uint32_t)(e + 127) << 23);
 }
-// Running maximum over eight scales (or biases) of a row as bf16 magnitudes, `up` added to the exponent of each.
-__device__ __forceinline__ uint32_t max_mag(uint4 v, uint32_t up, uint32_t m) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) m = __vmaxu2(m, (w[i] & 0x7fff7fffu) + up);
-    return m;
+// Running maximum over two scales (or biases) of a row as bf16 magnitudes, `up` added to the exponent of each.
+__device__ __forceinline__ uint32_t max_mag(uint32_t v, uint32_t up, uint32_t m) { return __vmaxu2(m, (v & 0x7fff7fffu) + up); }
+// f(word) for every 32-bit word of a row of scales (a multiple of 4 bytes), 16 bytes a load where the length allows.
+template <typename F>
+__device__ __forceinline__ void each_word_shared(uint32_t addr, uint32_t bytes, F&& f) {
+    if (bytes % 16 == 0) {
+        for (uint32_t i = 0; i < bytes; i += 16) {
+            const uint4 v = lds128(addr + i);
+            f(v.x); f(v.y); f(v.z); f(v.w);
+        }
+    } else {
+        for (uint32_t i = 0; i < bytes; i += 4) f(lds32(addr + i));
+    }
+}
+template <typename F>
+__device__ __forceinline__ void each_word_global(const uint8_t* p, int bytes, F&& f) {
+    if (bytes % 16 == 0) {
+        for (int i = 0; i < bytes; i += 16) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p + i));
+            f(v.x); f(v.y); f(v.z); f(v.w);
+        }
+    } else {
+        for (int i = 0; i < bytes; i += 4) f(__ldg(reinterpret_cast<const uint32_t*>(p + i)));
+    }
 }
 // The exponent k of the row's power of two: its largest |s| 2^bits or |b| comes to lie in [2^13, 2^14).
 __device__ __forceinline__ int row_shift(uint32_t mag2) { return 140 - (int)(max(mag2 & 0xffffu, mag2 >> 16) >> 7); }
@@ -514,13 +538,6 @@ __device__ __forceinline__ __half2 pow2_half2(int d) {
     return bits_h2(b | (b << 16));
 }
 
-// largest byte of n16 16-byte pieces
-__device__ __forceinline__ uint32_t max_byte(uint4 v, uint32_t m) {
-    m = __vmaxu4(m, v.x);
-    m = __vmaxu4(m, v.y);
-    m = __vmaxu4(m, v.z);
-    return __vmaxu4(m, v.w);
-}
 __device__ __forceinline__ uint32_t hmax_bytes(uint32_t m) {
     m = max(m & 0xffu, max((m >> 8) & 0xffu, max((m >> 16) & 0xffu, m >> 24)));
     return m;
@@ -538,7 +555,9 @@ __device__ __forceinline__ uint32_t hmax_bytes(uint32_t m) {
 // B200, both products: 8192 tokens over 256 experts of 2048 x 512, 4-bit 736 -> 580 us, 4096 tokens nvfp4 445 -> 356 us,
 // 1777 tokens 8-bit 417 -> 328 us, 16384 skewed tokens 2-bit 1303 -> 1032 us.  What bounds them now is the MMAs (M = 256,
 // N = 256: 128 cycles each, 512 of the 577 a K step takes in the first product) and the epilogue between tiles.
-template <bool SWIGLU, int FMT, bool TS, bool WIDE, bool XR, bool PAIR>
+// BF16: the rows leave rounded to bf16 (the second product alone).  A kernel of its own, since the epilogue is short of
+// registers: with the choice made at run time every call of the block lost 2 to 4 %.
+template <bool SWIGLU, int FMT, bool TS, bool WIDE, bool XR, bool PAIR, bool BF16>
 __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcParams& p, const TcMaps& maps) {
     static_assert(!PAIR || WIDE, "pairs of CTAs: wide tiles");
     static_assert(!WIDE || (TS && !XR), "wide tiles: tensor-memory operand, streamed activations");
@@ -667,11 +686,17 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                 const uint32_t bar = smem_u32(&bars->sfull[sbuf]);
                 const uint32_t dst = sc_base + (uint32_t)(sbuf * p.sc_bytes);
                 mbar_expect_tx(bar, (AFFINE ? 4u : 2u) * 64u * srow);
-                tma_load_2d(dst, &maps.s[mi0], 0, row0, bar);
-                tma_load_2d(dst + 64 * srow, &maps.s[mi1], 0, row1, bar);
+                // rows of scales lie one behind the other: 64 of them are one run of bytes, of any row length
+                const ExpertSet& S = a.set;
+                const QMat& m0 = SWIGLU ? (t.extra ? S.x_gate : S.gate) : (t.extra ? S.x_down : S.down);
+                const QMat& m1 = SWIGLU ? (t.extra ? S.x_up : S.up) : m0;
+                const size_t e_off = t.extra ? 0 : (size_t)t.expert * (SWIGLU ? S.gu_stride_s : S.dn_stride_s);
+                const size_t r0 = e_off + (size_t)t.ntile * (SWIGLU ? 64 : 128) * srow, r1 = SWIGLU ? r0 : r0 + 64 * (size_t)srow;
+                bulk_load(dst, m0.scales + r0, 64 * srow, bar);
+                bulk_load(dst + 64 * srow, m1.scales + r1, 64 * srow, bar);
                 if (AFFINE) {
-                    tma_load_2d(dst + 128 * srow, &maps.b[mi0], 0, row0, bar);
-                    tma_load_2d(dst + 192 * srow, &maps.b[mi1], 0, row1, bar);
+                    bulk_load(dst + 128 * srow, m0.biases + r0, 64 * srow, bar);
+                    bulk_load(dst + 192 * srow, m1.biases + r1, 64 * srow, bar);
                 }
             }
             __syncwarp();
@@ -725,10 +750,8 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                     const int srow = (t.K >> p.lg_group) * 2;
                     const size_t off = (t.extra ? 0 : (size_t)t.expert * estride) + (size_t)r_in * srow;
                     uint32_t mx = 0;
-                    for (int i = 0; i < srow; i += 16) {
-                        mx = max_mag(__ldg(reinterpret_cast<const uint4*>(m.scales + off + i)), (uint32_t)TBITS * 0x00800080u, mx);
-                        mx = max_mag(__ldg(reinterpret_cast<const uint4*>(m.biases + off + i)), 0u, mx);
-                    }
+                    each_word_global(m.scales + off, srow, [&](uint32_t v) { mx = max_mag(v, (uint32_t)TBITS * 0x00800080u, mx); });
+                    each_word_global(m.biases + off, srow, [&](uint32_t v) { mx = max_mag(v, 0u, mx); });
                     const int k = row_shift(mx);
                     return pow2_f32(-(k / 2)) * pow2_f32(-(k - k / 2));
                 }
@@ -737,13 +760,13 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                 const int srow = t.K >> 5;                          // one ue8m0 byte per 32 values
                 const uint8_t* sp = m.scales + (t.extra ? 0 : (size_t)t.expert * estride) + (size_t)r_in * srow;
                 uint32_t mx = 0;
-                for (int i = 0; i < srow; i += 16) mx = max_byte(__ldg(reinterpret_cast<const uint4*>(sp + i)), mx);
+                each_word_global(sp, srow, [&](uint32_t v) { mx = __vmaxu4(mx, v); });
                 return ue8m0_to_f32(hmax_bytes(mx));
             };
             // [lane group of 16][gate, up], or the weight rows 16 gs + 8 r8 + lane / 4 of the warp's 32; second product
             // with one weight row a lane (fp32 rows): [0]
             float rf[4] = {1.f, 1.f, 1.f, 1.f};
-            const bool frag_rows = !SWIGLU && WIDE && a.row_scale == nullptr && (a.out16 != nullptr || a.out_bf16 != nullptr);
+            const bool frag_rows = !SWIGLU && WIDE && a.row_scale == nullptr && (BF16 || a.out16 != nullptr);
             if (SWIGLU) {
 #pragma unroll
                 for (int gs = 0; gs < 2; ++gs) {
@@ -871,7 +894,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                                 for (int r8 = 0; r8 < 2; ++r8) {
                                     float x0 = __uint_as_float(v[4 * j + 2 * r8]), x1 = __uint_as_float(v[4 * j + 2 * r8 + 1]);
                                     if (!AFFINE || TWO) { x0 *= rf[2 * gs + r8]; x1 *= rf[2 * gs + r8]; }
-                                    if (a.out_bf16 != nullptr) {
+                                    if constexpr (BF16) {
                                         h[2 * gs + r8][j] = pack_bf16(x0, x1);
                                     } else {
                                         peak = fmaxf(peak, fmaxf(8 * j < n_ok ? fabsf(x0) : 0.f, 8 * j + 1 < n_ok ? fabsf(x1) : 0.f));
@@ -887,7 +910,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                         __syncwarp();
                     };
                     auto flush = [&](int c) {
-                        uint16_t* rows16 = a.out_bf16 != nullptr ? reinterpret_cast<uint16_t*>(a.out_bf16) : reinterpret_cast<uint16_t*>(a.out16);
+                        uint16_t* rows16 = BF16 ? reinterpret_cast<uint16_t*>(a.out_bf16) : reinterpret_cast<uint16_t*>(a.out16);
                         const int sl0 = (eh * 2 + c) * 64;
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
@@ -936,7 +959,15 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                     }
                     const size_t o0 = (size_t)(t.slot0 + c * 32) * a.set.n_in + col;
                     const int n_ok = t.rows - c * 32;
-                    if (a.out16 != nullptr && a.out_index != nullptr) {
+                    // (wide tiles: 16-bit rows without a weight per slot went out above)
+                    if constexpr (BF16) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 2) {
+                            const uint32_t h = pack_bf16(o[i], o[i + 1]);
+                            if (i < n_ok) st_global_u16(a.out_bf16 + o0 + (size_t)i * a.set.n_in, h);
+                            if (i + 1 < n_ok) st_global_u16(a.out_bf16 + o0 + (size_t)(i + 1) * a.set.n_in, h >> 16);
+                        }
+                    } else if (!WIDE && a.out16 != nullptr && a.out_index != nullptr) {
                         // rows scattered to the positions the caller names (expert parallelism: straight into the
                         // buffer the rows travel back in): one index per lane, handed round by shuffle
                         const int my = c * 32 + lane;
@@ -949,14 +980,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                             if (i < n_ok) st_global_u16(a.out16 + (size_t)r0 * a.set.n_in + col, h);
                             if (i + 1 < n_ok) st_global_u16(a.out16 + (size_t)r1 * a.set.n_in + col, h >> 16);
                         }
-                    } else if (a.out_bf16 != nullptr) {
-#pragma unroll
-                        for (int i = 0; i < 32; i += 2) {
-                            const uint32_t h = pack_bf16(o[i], o[i + 1]);
-                            if (i < n_ok) st_global_u16(a.out_bf16 + o0 + (size_t)i * a.set.n_in, h);
-                            if (i + 1 < n_ok) st_global_u16(a.out_bf16 + o0 + (size_t)(i + 1) * a.set.n_in, h >> 16);
-                        }
-                    } else if (a.out16 != nullptr) {
+                    } else if (!WIDE && a.out16 != nullptr) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 2) {
                             peak = fmaxf(peak, fmaxf(fabsf(o[i]), fabsf(o[i + 1])));
@@ -1003,16 +1027,14 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             int r_exp = 0;
             if (FMT == FMT_MXFP8) {
                 uint32_t mx = 0;
-                for (uint32_t i = 0; i < srow; i += 16) mx = max_byte(lds128(s_addr + i), mx);
+                each_word_shared(s_addr, srow, [&](uint32_t v) { mx = __vmaxu4(mx, v); });
                 r_exp = (int)hmax_bytes(mx);
             }
             float up0 = 1.f, up1 = 1.f;               // two-term weights: the row's 2^k, as two factors in fp32's range
             if (TWO) {
                 uint32_t mx = 0;
-                for (uint32_t i = 0; i < srow; i += 16) {
-                    mx = max_mag(lds128(s_addr + i), (uint32_t)TBITS * 0x00800080u, mx);
-                    mx = max_mag(lds128(b_addr + i), 0u, mx);
-                }
+                each_word_shared(s_addr, srow, [&](uint32_t v) { mx = max_mag(v, (uint32_t)TBITS * 0x00800080u, mx); });
+                each_word_shared(b_addr, srow, [&](uint32_t v) { mx = max_mag(v, 0u, mx); });
                 const int k = row_shift(mx);
                 up0 = pow2_f32(k / 2);
                 up1 = pow2_f32(k - k / 2);
@@ -1029,10 +1051,10 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                     using Tt = TwoTerm<TBITS>;
                     // the step's 64 codes of this row as a bit stream
                     uint32_t w[2 * TBITS];
-                    if (TBITS == 6 || TBITS == 4) {
+                    if (TBITS % 2 == 0) {
 #pragma unroll
                         for (int c = 0; c < TBITS / 2; ++c) {
-                            const uint4 v = lds128(stage + q_off + (((uint32_t)c ^ (TBITS == 4 ? swz : 0u)) << 4));
+                            const uint4 v = lds128(stage + q_off + (((uint32_t)c ^ (TBITS == 4 || TBITS == 8 ? swz : 0u)) << 4));
                             w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
                         }
                     } else {
@@ -1123,16 +1145,16 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
     if (tid == 0 && bars->abort && a.status != nullptr) atomicExch(a.status, 3);
 }
 
-template <bool SWIGLU, int FMT, bool TS, bool WIDE, bool XR>
+template <bool SWIGLU, int FMT, bool TS, bool WIDE, bool XR, bool BF16 = false>
 __global__ void __launch_bounds__(kThreadsTc, 1)
 prefill_tc_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__ TcMaps maps) {
-    prefill_tc_body<SWIGLU, FMT, TS, WIDE, XR, false>(a, p, maps);
+    prefill_tc_body<SWIGLU, FMT, TS, WIDE, XR, false, BF16>(a, p, maps);
 }
 
-template <bool SWIGLU, int FMT>
+template <bool SWIGLU, int FMT, bool BF16 = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsTc, 1)
 prefill_pair_kernel(const GroupedArgs a, const TcParams p, const __grid_constant__ TcMaps maps) {
-    prefill_tc_body<SWIGLU, FMT, true, true, false, true>(a, p, maps);
+    prefill_tc_body<SWIGLU, FMT, true, true, false, true, BF16>(a, p, maps);
 }
 
 }  // namespace
@@ -1148,7 +1170,8 @@ int fmt_index(const QFormat& f) {
 
 // The two-term form of a format, or -1.
 int two_term_index(const QFormat& f) {
-    return f.mode == IMX_MODE_AFFINE && f.bits >= 3 && f.bits <= 6 ? FMT_T3 + f.bits - 3 : -1;
+    if (f.mode != IMX_MODE_AFFINE) return -1;
+    return f.bits == 8 ? FMT_T8 : (f.bits >= 2 && f.bits <= 6 ? FMT_T2 + f.bits - 2 : -1);
 }
 
 int log2_exact(int v) {
@@ -1164,21 +1187,15 @@ bool k_ok(int K, const QFormat& f) {
     const size_t sr = scale_row(K, f);
     return sr % 16 == 0 && K / f.group <= 256;
 }
+// ... and what the kernels themselves need of it (whole 32-bit words)
+bool k_ok_any(int K, const QFormat& f) { return K % kTileK == 0 && K % f.group == 0 && scale_row(K, f) % 4 == 0 && K / f.group <= 256; }
 
-// packed codes + scales (+ biases) maps of one stacked quantized matrix [rows, K]
-int make_q_maps(const QMat& m, size_t rows, int K, const QFormat& f, int fmt, CUtensorMap* w, CUtensorMap* sc, CUtensorMap* bi) {
+// map of the packed codes of one stacked quantized matrix [rows, K]
+int make_q_map(const QMat& m, size_t rows, int K, const QFormat& f, int fmt, CUtensorMap* w) {
     const int qrow = q_row_bytes(fmt);
     const size_t row_bytes = packed_row_bytes(K, f.bits);
     const int swz = qrow == 64 ? 64 : (qrow == 32 ? 32 : 0);
     IMX_TRY(make_tensor_map_2d(m.w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, rows, row_bytes, row_bytes, qrow, 64, false, w, false, swz));
-    const int groups = K / f.group;
-    if (f.mode == IMX_MODE_AFFINE) {
-        IMX_TRY(make_tensor_map_2d(m.scales, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, rows, groups, (size_t)groups * 2, groups, 64, false, sc));
-        IMX_TRY(make_tensor_map_2d(m.biases, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, rows, groups, (size_t)groups * 2, groups, 64, false, bi));
-    } else {
-        IMX_TRY(make_tensor_map_2d(m.scales, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, rows, groups, (size_t)groups, groups, 64, false, sc));
-        *bi = *sc;
-    }
     return IMX_OK;
 }
 
@@ -1189,11 +1206,14 @@ int configure() {
     constexpr int kSmem = (int)kSmemMost;
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_pair_kernel<true, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_pair_kernel<false, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_pair_kernel<false, FMT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     if constexpr (two_term(FMT)) {
         IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
         IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
         return IMX_OK;
     } else {
+    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
@@ -1216,6 +1236,14 @@ struct Plan {
 template <int FMT>
 int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, const TcMaps& mgu, const TcMaps& mdn, int sms,
                cudaStream_t stream, cudaEvent_t mid) {
+    if (a.out_bf16 != nullptr) {
+        if (dn.pair) prefill_pair_kernel<false, FMT, true><<<sms & ~1, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        else if (dn.wide) prefill_tc_kernel<false, FMT, true, true, false, true><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        else if constexpr (!two_term(FMT)) prefill_tc_kernel<false, FMT, true, false, false, true><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        IMX_LAUNCHED();
+        IMX_CHECK_CUDA(cudaGetLastError());
+        return IMX_OK;
+    }
     if constexpr (two_term(FMT)) {
         if (!a.second_only) {
             if (gu.pair) prefill_pair_kernel<true, FMT><<<sms & ~1, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
@@ -1296,16 +1324,20 @@ extern "C" IMX_API int imx_debug_tc_prof(unsigned long long* out32) {
 }
 #endif
 
-bool prefill_tc_supported(const ExpertSet& s, bool second_only) {
+static bool tc_supported(const ExpertSet& s, bool second_only, bool (*ok)(int, const QFormat&)) {
     const QFormat& f = s.fmt;
     if (fmt_index(f) < 0) return false;
     if (log2_exact(f.group) < 0 || f.group > 128 || f.group < 16) return false;
     if (f.mode == IMX_MODE_AFFINE && f.group < 32) return false;
     if (s.n_in % 128 || s.n_mid % 64) return false;
     // the second product alone never reduces over n_in (a plain quantized matmul with any number of output rows)
-    if ((!second_only && !k_ok(s.n_in, f)) || !k_ok(s.n_mid, f)) return false;
-    if (s.has_extra && (s.x_mid % 64 || !k_ok(s.x_mid, f))) return false;
+    if ((!second_only && !ok(s.n_in, f)) || !ok(s.n_mid, f)) return false;
+    if (s.has_extra && (s.x_mid % 64 || !ok(s.x_mid, f))) return false;
     return true;
+}
+bool prefill_tc_supported(const ExpertSet& s, bool second_only) { return tc_supported(s, second_only, k_ok); }
+bool tc_rows32_supported(const ExpertSet& s) {
+    return (s.fmt.mode == IMX_MODE_MXFP8 || s.fmt.mode == IMX_MODE_NVFP4) && tc_supported(s, false, k_ok_any);
 }
 
 // Do the weight tiles of a unit pair up (64 gate and 64 up rows, 128 output rows a tile)?
@@ -1315,10 +1347,10 @@ static bool second_even(const ExpertSet& s) { return s.n_in % 256 == 0; }
 bool two_term_supported(const ExpertSet& s, bool second_only) {
     const QFormat& f = s.fmt;
     const int fmt = two_term_index(f);
-    if (fmt < 0 || (f.bits == 4 && f.group != 32)) return false;
-    if (s.n_in % 128) return false;
+    if (fmt < 0 || log2_exact(f.group) < 0 || f.group < 32 || f.group > 128) return false;
+    if (s.n_in % 128 || (!second_only && s.n_mid % 64) || (s.has_extra && s.x_mid % 64)) return false;
     // packed rows advance in whole 16-byte pieces (the pitch a tiled copy needs)
-    auto ok = [&](int K) { return k_ok(K, f) && packed_row_bytes(K, f.bits) % 16 == 0; };
+    auto ok = [&](int K) { return k_ok_any(K, f) && packed_row_bytes(K, f.bits) % 16 == 0; };
     if ((!second_only && !ok(s.n_in)) || !ok(s.n_mid) || (s.has_extra && !ok(s.x_mid))) return false;
     const int mid_max = s.has_extra && s.x_mid > s.n_mid ? s.x_mid : s.n_mid;
     Plan p;
@@ -1326,8 +1358,8 @@ bool two_term_supported(const ExpertSet& s, bool second_only) {
            wide_plan(f, fmt, mid_max, mid_max, second_even(s), 0, &p);
 }
 
-// What the copy engine asks of the matrices' addresses (the scalar kernel takes any 16 / 4-byte aligned tensor).
-bool two_term_aligned(const ExpertSet& s, bool second_only) {
+// What the copy engine asks of the matrices' addresses (the other kernels take any 16 / 4-byte aligned tensor).
+bool tc_aligned(const ExpertSet& s, bool second_only) {
     auto ok = [](const QMat& m) { return (((uintptr_t)m.w | (uintptr_t)m.scales | (uintptr_t)m.biases) % 16) == 0; };
     if (!ok(s.down) || (!second_only && !(ok(s.gate) && ok(s.up)))) return false;
     return !s.has_extra || (ok(s.x_down) && (second_only || (ok(s.x_gate) && ok(s.x_up))));
@@ -1337,10 +1369,12 @@ bool two_term_aligned(const ExpertSet& s, bool second_only) {
 // tensor-memory operand, 128-slot tiles and streamed activations everywhere, 2 = as 1 with the dequantized
 // tile in shared memory (1, 2: cross-checks).
 int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid, int variant) {
-    IMX_REQUIRE(variant == 3 ? two_term_supported(a.set, a.second_only != 0) : prefill_tc_supported(a.set, a.second_only != 0),
+    IMX_REQUIRE(variant == 3 ? two_term_supported(a.set, a.second_only != 0)
+                : (variant == 0 && a.out16 == nullptr && tc_rows32_supported(a.set)) || prefill_tc_supported(a.set, a.second_only != 0),
                 "prefill path: format/shape not supported");
     IMX_REQUIRE((a.row_index == nullptr || a.xs != nullptr || a.second_only) && a.n_slots > 0,
                 "prefill path: slot-ordered activation buffer missing");
+    IMX_REQUIRE(tc_aligned(a.set, a.second_only != 0), "prefill path: weights, scales and biases must be 16-byte aligned");
     if (a.max_units == 0) return IMX_OK;
     const ExpertSet& s = a.set;
     const QFormat& f = s.fmt;
@@ -1358,10 +1392,12 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
         IMX_TRY(configure<FMT_A2>());
         IMX_TRY(configure<FMT_MXFP8>());
         IMX_TRY(configure<FMT_NVFP4>());
+        IMX_TRY(configure<FMT_T2>());
         IMX_TRY(configure<FMT_T3>());
         IMX_TRY(configure<FMT_T4>());
         IMX_TRY(configure<FMT_T5>());
         IMX_TRY(configure<FMT_T6>());
+        IMX_TRY(configure<FMT_T8>());
         device_mark_setup(di.ordinal, kSetupPrefillTc);
     }
 
@@ -1369,6 +1405,8 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
         return make_plan(f, fmt, K_max, K_min, wide, xr, ts, out);
     };
     Plan gu = {}, dn = {};
+    IMX_REQUIRE(a.out16 == nullptr || a.row_scale == nullptr, "prefill path: fp16 rows carry no weight per slot");
+    IMX_REQUIRE(a.out_bf16 == nullptr || (a.second_only && variant != 1 && variant != 2), "prefill path: bf16 rows belong to the second product alone");
     const int epi_second = a.out16 != nullptr || a.out_bf16 != nullptr ? kEpiSecond : 0;
     if (variant == 3) {
         IMX_REQUIRE((a.second_only || wide_plan(f, fmt, s.n_in, s.n_in, first_even(s), kEpiFirst, &gu)) &&
@@ -1379,7 +1417,8 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
             IMX_REQUIRE(plan(s.n_in, s.n_in, false, false, &gu), "prefill path: sizes exceed shared memory");
         // second product: 256-slot tiles with streamed activations as well (c3: 276 us against 377 us with 128-slot
         // tiles and the activation panel resident, one CTA a tile); the resident panel where the wide stages do not fit
-        if (!(variant == 0 && (wide_plan(f, fmt, mid_max, mid_min, second_even(s), epi_second, &dn) || plan(mid_max, mid_min, false, true, &dn))))
+        if (!(variant == 0 && (wide_plan(f, fmt, mid_max, mid_min, second_even(s), epi_second, &dn) ||
+                               (a.out_bf16 == nullptr && plan(mid_max, mid_min, false, true, &dn)))))
             IMX_REQUIRE(plan(mid_max, mid_min, false, false, &dn), "prefill path: sizes exceed shared memory");
     }
     gu.p.nt_r = s.n_mid / 64;
@@ -1407,19 +1446,18 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
     IMX_TRY(make_tensor_map_2d(a.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (size_t)a.n_slots, (size_t)mid_max, (size_t)a.act_stride * 2,
                                kTileK, 128, true, &mdn.x));
     // routed experts: gate and up rows live in one stacked matrix [E*2I, H]; down in [E*H, I]
-    if (!a.second_only) IMX_TRY(make_q_maps(s.gate, (size_t)s.num_experts * 2 * s.n_mid, s.n_in, f, fmt, &mgu.w[0], &mgu.s[0], &mgu.b[0]));
-    IMX_TRY(make_q_maps(s.down, (size_t)s.num_experts * s.n_in, s.n_mid, f, fmt, &mdn.w[0], &mdn.s[0], &mdn.b[0]));
+    if (!a.second_only) IMX_TRY(make_q_map(s.gate, (size_t)s.num_experts * 2 * s.n_mid, s.n_in, f, fmt, &mgu.w[0]));
+    IMX_TRY(make_q_map(s.down, (size_t)s.num_experts * s.n_in, s.n_mid, f, fmt, &mdn.w[0]));
+    mgu.w[1] = mgu.w[2] = mgu.w[0];
+    mdn.w[1] = mdn.w[0];
     if (s.has_extra) {
         if (!a.second_only) {
-            IMX_TRY(make_q_maps(s.x_gate, (size_t)s.x_mid, s.n_in, f, fmt, &mgu.w[1], &mgu.s[1], &mgu.b[1]));
-            IMX_TRY(make_q_maps(s.x_up, (size_t)s.x_mid, s.n_in, f, fmt, &mgu.w[2], &mgu.s[2], &mgu.b[2]));
+            IMX_TRY(make_q_map(s.x_gate, (size_t)s.x_mid, s.n_in, f, fmt, &mgu.w[1]));
+            IMX_TRY(make_q_map(s.x_up, (size_t)s.x_mid, s.n_in, f, fmt, &mgu.w[2]));
         }
-        IMX_TRY(make_q_maps(s.x_down, (size_t)s.n_in, s.x_mid, f, fmt, &mdn.w[1], &mdn.s[1], &mdn.b[1]));
-    } else {
-        mgu.w[1] = mgu.w[2] = mgu.w[0]; mgu.s[1] = mgu.s[2] = mgu.s[0]; mgu.b[1] = mgu.b[2] = mgu.b[0];
-        mdn.w[1] = mdn.w[0]; mdn.s[1] = mdn.s[0]; mdn.b[1] = mdn.b[0];
+        IMX_TRY(make_q_map(s.x_down, (size_t)s.n_in, s.x_mid, f, fmt, &mdn.w[1]));
     }
-    mdn.w[2] = mdn.w[1]; mdn.s[2] = mdn.s[1]; mdn.b[2] = mdn.b[1];
+    mdn.w[2] = mdn.w[1];
 
     switch (fmt) {
         case FMT_A4: return launch_fmt<FMT_A4>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
@@ -1427,6 +1465,8 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
         case FMT_A2: return launch_fmt<FMT_A2>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
         case FMT_MXFP8: return launch_fmt<FMT_MXFP8>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
         case FMT_NVFP4: return launch_fmt<FMT_NVFP4>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
+        case FMT_T2: return launch_fmt<FMT_T2>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
+        case FMT_T8: return launch_fmt<FMT_T8>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
         case FMT_T3: return launch_fmt<FMT_T3>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
         case FMT_T4: return launch_fmt<FMT_T4>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
         case FMT_T5: return launch_fmt<FMT_T5>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
