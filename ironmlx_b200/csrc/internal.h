@@ -176,7 +176,7 @@ constexpr int kPrefillUnitRows = 256;
 bool prefill_tc_supported(const ExpertSet& s, bool second_only = false);
 int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid = nullptr, int variant = 0);
 // The same kernels with the weight as a two-term fp16 sum, for the formats whose weights stay in 32 bits: affine
-// 3/5/6-bit and 4-bit in groups of 32.  kPathTwoTerm is what pick_path answers for them (never a caller's request).
+// 3/5/6-bit and groups of 32 at any size, the other widths between decode and prefill sizes.  kPathTwoTerm is what pick_path answers for them (never a caller's request).
 constexpr int kPathTwoTerm = 100;
 // The tensor-core kernels with fp32 expert rows, for batches whose rows the decode kernels keep in fp32 (mxfp8, nvfp4).
 constexpr int kPathTcRows32 = 101;

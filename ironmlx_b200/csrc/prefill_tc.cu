@@ -444,16 +444,16 @@ struct Dequant<FMT_NVFP4> {
 };
 
 // ── two-term weights ────────────────────────────────────────────────────────
-// The formats no 16-bit kernel served before (affine 3/5/6-bit, and 4-bit in groups of 32) had their weights in fp32
-// in the scalar kernel.  One fp16 rounding of s * q + b would be a loss, so the MMA gets the weight as a sum of two
+// The formats no 16-bit kernel serves (affine 3/5/6-bit, groups of 32) had their weights in fp32 in the scalar kernel, and
+// the decode kernels keep affine weights exact.  One fp16 rounding of s * q + b would be a loss, so the MMA gets the weight as a sum of two
 // fp16 terms, hi + lo, good to 22 bits, with two MMAs per 16 values: the tile of A is 64 tensor-memory columns per
 // K step.  Everything is exact but the last rounding of lo:
 //   p = rn(q * s), e = q * s - p           exact: s is a bf16 value (8 bits), q has at most 6
 //   hi = rn(p + b), lo = rn(e + err)       err = the rounding error of p + b (two-sum)
 // fp16's range is met by a power of two 2^k per weight row, from the row's largest |s| 2^bits or |b|, taken back in
 // the epilogue (fp32).  Measured on a B200 against the scalar kernels, 1000 tokens over 256 experts of 2048 x 512, 6-bit:
-// both products 5.65 ms -> 0.52 ms (the block 5.74 -> 0.57 ms); what bounds it now is the MMAs' issue (eight per K step
-// whatever their N) beside the dequantization, two thirds of a K step's time.  Codes are pulled out in pairs (a, a + D) of a window of the bit stream, so that the second
+// both products 5.65 ms -> 0.48 ms (the block 5.73 -> 0.54 ms); what bounds it now is the dequantization: twelve
+// half-precision operations a pair of values in eight warps, two thirds of a K step's time.  Codes are pulled out in pairs (a, a + D) of a window of the bit stream, so that the second
 // one lands in the upper half-word HS bits up (that factor goes into its copy of the scale); codes of a block of 16
 // that have no partner at that distance pair with their neighbour.
 template <int BITS>
