@@ -766,7 +766,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             // [lane group of 16][gate, up], or the weight rows 16 gs + 8 r8 + lane / 4 of the warp's 32; second product
             // with one weight row a lane (fp32 rows): [0]
             float rf[4] = {1.f, 1.f, 1.f, 1.f};
-            const bool frag_rows = !SWIGLU && WIDE && a.row_scale == nullptr && (BF16 || a.out16 != nullptr);
+            const bool frag_rows = !SWIGLU && WIDE && p.epi_bytes != 0;
             if (SWIGLU) {
 #pragma unroll
                 for (int gs = 0; gs < 2; ++gs) {
@@ -1309,12 +1309,16 @@ bool make_plan(const QFormat& f, int fmt, int K_max, int K_min, bool wide, bool 
 }
 
 // Wide tiles of one product: in pairs of CTAs where the weight tiles of a unit pair up, else one CTA each.  16-bit
-// results are turned round in shared memory (first product 48, second 80 bytes a slot; fp32 rows need none).
+// results are turned round in shared memory (first product 48, second 80 bytes a slot).
 constexpr int kEpiFirst = 48, kEpiSecond = 80;
 bool wide_plan(const QFormat& f, int fmt, int K_max, int K_min, bool even, int epi_row, Plan* out) {
     return (even && make_plan(f, fmt, K_max, K_min, true, false, true, out, true, epi_row)) ||
            make_plan(f, fmt, K_max, K_min, true, false, true, out, false, epi_row);
 }
+
+// Bytes a slot of the second product's transposing buffer: 16-bit rows without a factor per slot go through it, fp32
+// rows and rows with a factor (those of every two-term matrix) leave as single values.
+int second_epi(bool rows16, bool scaled) { return rows16 && !scaled ? kEpiSecond : 0; }
 
 }  // namespace
 
@@ -1355,7 +1359,7 @@ bool two_term_supported(const ExpertSet& s, bool second_only) {
     const int mid_max = s.has_extra && s.x_mid > s.n_mid ? s.x_mid : s.n_mid;
     Plan p;
     return (second_only || wide_plan(f, fmt, s.n_in, s.n_in, first_even(s), kEpiFirst, &p)) &&
-           wide_plan(f, fmt, mid_max, mid_max, second_even(s), 0, &p);
+           wide_plan(f, fmt, mid_max, mid_max, second_even(s), second_epi(second_only, true), &p);
 }
 
 // What the copy engine asks of the matrices' addresses (the other kernels take any 16 / 4-byte aligned tensor).
@@ -1407,7 +1411,7 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
     Plan gu = {}, dn = {};
     IMX_REQUIRE(a.out16 == nullptr || a.row_scale == nullptr, "prefill path: fp16 rows carry no weight per slot");
     IMX_REQUIRE(a.out_bf16 == nullptr || (a.second_only && variant != 1 && variant != 2), "prefill path: bf16 rows belong to the second product alone");
-    const int epi_second = a.out16 != nullptr || a.out_bf16 != nullptr ? kEpiSecond : 0;
+    const int epi_second = second_epi(a.out16 != nullptr || a.out_bf16 != nullptr, a.row_scale != nullptr);
     if (variant == 3) {
         IMX_REQUIRE((a.second_only || wide_plan(f, fmt, s.n_in, s.n_in, first_even(s), kEpiFirst, &gu)) &&
                         wide_plan(f, fmt, mid_max, mid_min, second_even(s), epi_second, &dn),

@@ -53,6 +53,15 @@ def test_linear(cuda, bits, group, m, in_dim, out_dim):
     _check(layer.forward_with_stream(x), x, wd, in_dim)
 
 
+@pytest.mark.parametrize("bits,group,in_dim", [(6, 64, 9728), (6, 64, 11008), (3, 64, 8192), (5, 32, 5120), (4, 32, 4096)])
+@pytest.mark.parametrize("m,out_dim", [(3, 384), (20, 512)])
+def test_linear_of_long_rows(cuda, bits, group, in_dim, m, out_dim):
+    """Rows of scales that leave little shared memory beside them, with weight tiles that pair up (512) and do not (384)."""
+    layer, wd, gen = _layer(cuda, out_dim, in_dim, bits, group, 11)
+    x = torch.randn(m, in_dim, generator=gen, device=cuda).to(torch.bfloat16)
+    _check(layer.forward_with_stream(x), x, wd, in_dim)
+
+
 @pytest.mark.parametrize("bits,group", [(6, 64), (3, 64)])
 @pytest.mark.parametrize("x_scale,w_scale", [(1e20, 1e-12), (1e-25, 1e10), (1e-3, 1e-6), (70000.0, 3.0)])
 def test_linear_outside_the_range_of_fp16(cuda, bits, group, x_scale, w_scale):
