@@ -210,8 +210,15 @@ int launch_tile(const void* x, int n, int H, const void* Wr, const float* logit_
 
 }  // namespace
 
+// A tile takes all K steps one after the other whatever the batch (15 us at a hidden size of 512, 29 at 2048, 73 at 9728),
+// the cluster-per-token kernel's time grows with the tokens and, less, with the experts; it serves the batches that this
+// one would spread over a few CTAs.  Both on a B200, cluster / this one, us: 16 experts of 512, 256 tokens 9.2 / 15.2, 400
+// 13.3 / 14.6, 700 17.4 / 15.4; 16 of 2048, 700 tokens 22.7 / 28.6, 1024 28.5 / 28.7, 1400 33.8 / 28.8; 60 of 1024, 256 tokens
+// 14.5 / 18.3, 400 20.4 / 18.3; 60 of 2048, 400 tokens 26.4 / 30.8, 700 34.9 / 30.9.
+static bool enough_tokens(int n, int H, int E) { return (long)n * (E + 40) >= (H <= 1024 ? 30000L : 52000L); }
+
 bool route_tc_supported(const void* x, int n, int H, const void* Wr, int E, const void* x16, const Order16& order) {
-    return n >= 256 && H % kRtK == 0 && E <= kRtMaxExperts && (((uintptr_t)x | (uintptr_t)Wr | (uintptr_t)x16) % 16) == 0 &&
+    return n >= 256 && enough_tokens(n, H, E) && H % kRtK == 0 && E <= kRtMaxExperts && (((uintptr_t)x | (uintptr_t)Wr | (uintptr_t)x16) % 16) == 0 &&
            order_bits(order) >= 0;
 }
 

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,experts,hidden,k,shared,norm,bias", [
-    (257, 16, 512, 4, False, True, False),      # one accumulator, a single token in the last tile
+    (545, 16, 512, 4, False, True, False),      # one accumulator, a single token in the last tile
     (300, 72, 192, 8, True, False, True),       # experts that are no multiple of 32, three K steps
     (1031, 128, 1024, 4, True, True, False),    # the largest single accumulator
     (1024, 160, 64, 6, True, True, True),       # two, the second one short; one K step
@@ -42,3 +42,17 @@ def test_route(cuda, n, experts, hidden, k, shared, norm, bias):
     if shared:
         z = x.double() @ sg.double().T
         assert ((gate.double() - torch.sigmoid(z)[:, 0]).abs() <= eps + 2.0 ** -20).all()
+
+
+@pytest.mark.parametrize("n,experts,hidden", [(300, 16, 512), (400, 60, 2048), (900, 8, 2048)])
+def test_few_tokens_and_experts_stay_on_the_kernel_per_token(cuda, n, experts, hidden):
+    """Batches that would be a few tiles of the tensor-core router run on the kernel that takes a cluster per token, as
+    batches below 256 tokens do: the same sums in the same order, hence the same bits for the same token."""
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(n)
+    x = torch.randn(n, hidden, generator=gen, device=cuda).to(torch.bfloat16)
+    w = (torch.randn(experts, hidden, generator=gen, device=cuda) * 0.1).to(torch.bfloat16)
+    st = CudaStages(cuda)
+    idx, wt = (t.clone() for t in st.route(x, w, None, 4, True, None)[:2])
+    small = st.route(x[:255].contiguous(), w, None, 4, True, None)
+    assert torch.equal(idx[:255], small[0]) and torch.equal(wt[:255], small[1])
