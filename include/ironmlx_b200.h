@@ -344,7 +344,8 @@ IMX_API int imx_quantized_matmul(const void* x, int m, const imx_qtensor* w, int
  * contraction, so the call runs that kernel alone as a one-expert problem -- the tensor-map decode
  * kernel for few rows, the tcgen05 kernel from 32 rows up -- and falls back to the kernel above for
  * shapes neither takes.  `QuantizedLinear::forward_with_stream` (mlx/src/nn/linear.rs:51-63) with
- * caller-provided scratch (zero-filled once, 256-byte aligned). */
+ * caller-provided scratch (zero-filled once, 256-byte aligned).  y may start at any bf16 value; from 32 rows up,
+ * rows that start on a multiple of 16 bytes are written fastest. */
 IMX_API int imx_quantized_matmul_scratch_bytes(int m, int n_out, int in, int group_size, int bits, int mode,
                                        size_t* bytes);
 IMX_API int imx_quantized_matmul_ws(const void* x, int m, const imx_qtensor* w, int n_out, int in, int group_size,

@@ -18,6 +18,7 @@
 // from the caller.
 #include "internal.h"
 #include "route_common.cuh"
+#include "../../include/ironmlx_b200_testing.h"
 
 namespace imx {
 
@@ -295,8 +296,12 @@ int imx_quantized_matmul_ws(const void* x, int m, const imx_qtensor* w, int n_ou
     cudaStream_t stream = (cudaStream_t)stream_;
     ExpertSet set;
     IMX_TRY(qmm_set(*w, n_out, in, f, &set));
-    const int path = ((uintptr_t)w->w % 16 == 0 && (uintptr_t)w->scales % 16 == 0 && (w->biases == nullptr || (uintptr_t)w->biases % 16 == 0))
-                         ? qmm_path(set, m) : IMX_PATH_GENERIC;
+    IMX_REQUIRE((uintptr_t)y % 2 == 0, "quantized_matmul: y must be aligned to its bf16 values");
+    int path = ((uintptr_t)w->w % 16 == 0 && (uintptr_t)w->scales % 16 == 0 && (w->biases == nullptr || (uintptr_t)w->biases % 16 == 0))
+                   ? qmm_path(set, m) : IMX_PATH_GENERIC;
+    // the products store straight into y: the tensor-map decode kernel in pairs, the others as single values where y
+    // does not allow more (the tensor-core kernels look for themselves)
+    if (path == IMX_PATH_DECODE && decode_tmap_supported(set) && (uintptr_t)y % 4 != 0) path = IMX_PATH_DECODE_REGS;
     if (path == IMX_PATH_GENERIC)      // no expert kernel takes this shape: the scalar kernel
         return imx_quantized_matmul(x, m, w, n_out, in, 1, group_size, bits, mode, y, stream_);
     const OneWs ws = carve_one(m, in, 0, n_out, scratch);

@@ -1316,9 +1316,10 @@ bool wide_plan(const QFormat& f, int fmt, int K_max, int K_min, bool even, int e
            make_plan(f, fmt, K_max, K_min, true, false, true, out, false, epi_row);
 }
 
-// Bytes a slot of the second product's transposing buffer: 16-bit rows without a factor per slot go through it, fp32
-// rows and rows with a factor (those of every two-term matrix) leave as single values.
-int second_epi(bool rows16, bool scaled) { return rows16 && !scaled ? kEpiSecond : 0; }
+// Bytes a slot of the second product's transposing buffer: 16-bit rows without a factor per slot go through it to
+// 16-byte stores, fp32 rows, rows with a factor (those of every two-term matrix) and rows that do not start on a
+// multiple of 16 bytes leave as single values.
+int second_epi(const void* rows16, bool scaled) { return rows16 != nullptr && !scaled && (uintptr_t)rows16 % 16 == 0 ? kEpiSecond : 0; }
 
 }  // namespace
 
@@ -1359,7 +1360,7 @@ bool two_term_supported(const ExpertSet& s, bool second_only) {
     const int mid_max = s.has_extra && s.x_mid > s.n_mid ? s.x_mid : s.n_mid;
     Plan p;
     return (second_only || wide_plan(f, fmt, s.n_in, s.n_in, first_even(s), kEpiFirst, &p)) &&
-           wide_plan(f, fmt, mid_max, mid_max, second_even(s), second_epi(second_only, true), &p);
+           wide_plan(f, fmt, mid_max, mid_max, second_even(s), second_epi(nullptr, true), &p);
 }
 
 // What the copy engine asks of the matrices' addresses (the other kernels take any 16 / 4-byte aligned tensor).
@@ -1411,7 +1412,8 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
     Plan gu = {}, dn = {};
     IMX_REQUIRE(a.out16 == nullptr || a.row_scale == nullptr, "prefill path: fp16 rows carry no weight per slot");
     IMX_REQUIRE(a.out_bf16 == nullptr || (a.second_only && variant != 1 && variant != 2), "prefill path: bf16 rows belong to the second product alone");
-    const int epi_second = second_epi(a.out16 != nullptr || a.out_bf16 != nullptr, a.row_scale != nullptr);
+    IMX_REQUIRE((uintptr_t)a.out16 % 16 == 0, "prefill path: fp16 rows must be 16-byte aligned");
+    const int epi_second = second_epi(a.out_bf16 != nullptr ? (const void*)a.out_bf16 : a.out16, a.row_scale != nullptr);
     if (variant == 3) {
         IMX_REQUIRE((a.second_only || wide_plan(f, fmt, s.n_in, s.n_in, first_even(s), kEpiFirst, &gu)) &&
                         wide_plan(f, fmt, mid_max, mid_min, second_even(s), epi_second, &dn),

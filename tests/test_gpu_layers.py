@@ -86,3 +86,31 @@ def test_fusing_experts_with_different_tensor_scales_is_refused(cuda):
     b.global_scale = (a.global_scale or 1.0) * 2
     with pytest.raises(_lib.IronMLXError):
         nn.FusedExperts.from_experts([nn.Expert(a, a, a), nn.Expert(b, b, b)])
+
+
+@pytest.mark.parametrize("mode,bits,group,m", [("affine", 4, 64, 40), ("affine", 4, 64, 3), ("affine", 8, 64, 3), ("nvfp4", 4, 16, 3),
+                                               ("mxfp8", 8, 32, 200), ("affine", 6, 64, 40), ("affine", 4, 64, 5)])
+@pytest.mark.parametrize("at", [1, 2, 4])
+def test_quantized_linear_into_rows_at_any_value(cuda, mode, bits, group, m, at):
+    """`imx_quantized_matmul_ws` with y at 2, 4 and 8 bytes past a multiple of 16: the values of the aligned call (the
+    4-bit decode kernel that takes odd addresses adds in another order: one step of bf16), nothing around them."""
+    import ctypes as C
+    n_in, n_out = (512, 384) if m == 5 else (512, 1024)
+    ql = q_to_device(_qlinear(n_out, n_in, mode, bits, group, seed=17), cuda)
+    x = t_bf16(round_bf16(normal(18, "x", (m, n_in))), cuda)
+    want = ql.forward_with_stream(x)
+    buf = torch.full((m * n_out + 16,), 7.0, dtype=torch.bfloat16, device=cuda)
+    nb, qt, lib = C.c_size_t(0), ql.qtensor(), _lib.lib()
+    fmt = (group, bits, _lib.MODE[mode])
+    _lib.check(lib.imx_quantized_matmul_scratch_bytes(m, n_out, n_in, *fmt, C.byref(nb)))
+    scratch = torch.zeros(nb.value, dtype=torch.uint8, device=cuda)
+    _lib.check(lib.imx_quantized_matmul_ws(x.data_ptr(), m, C.byref(qt), n_out, n_in, *fmt, buf.data_ptr() + 2 * at,
+                                           scratch.data_ptr(), nb.value, torch.cuda.current_stream().cuda_stream))
+    got = buf[at:at + m * n_out].view(m, n_out)
+    assert (buf[:at] == 7).all() and (buf[at + m * n_out:] == 7).all()
+    if (mode, bits, m, at) == ("affine", 4, 3, 1):
+        assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + 1e-6).all()
+    else:
+        assert torch.equal(got, want)
+    assert lib.imx_quantized_matmul_ws(x.data_ptr(), m, C.byref(qt), n_out, n_in, *fmt, buf.data_ptr() + 1,
+                                       scratch.data_ptr(), nb.value, torch.cuda.current_stream().cuda_stream) == _lib.ERR_INVALID
