@@ -32,21 +32,56 @@ namespace {
 // rounding in the product's epilogue instead of a combine launch over fp32 rows: 777 rows 2048 -> 8192 56 -> 36 us, 6 rows
 // 2048 -> 152064 57 -> 51 us.  Block m: the identity slot order, the work units of the single expert (balanced,
 // at most unit_rows slots each) and cleared scheduler words.
-// row_scale: any bf16 row fits fp16 once its largest magnitude is brought into [2^14, 2^15) by a power of two, which
-// the output gets back: row_scale = 2^-k.  Rows of zeros and rows with infinities or NaNs stay as they are.
+// SCALED: any bf16 row fits fp16 once its largest magnitude is brought into [2^14, 2^15) by a power of two, which
+// the output gets back: row_scale = 2^-k.  Rows of zeros and rows with NaNs stay as they are.  A row with infinities would
+// meet weights split into two terms, inf * hi + inf * lo, which is NaN wherever the signs differ: its products, infinities
+// by the sign of the weights that meet one (NaN for a zero or opposite ones), are written here, and a NaN for its factor
+// tells the product's epilogue to leave them.
 constexpr int kPrepThreads = 256;
 
-__global__ void __launch_bounds__(kPrepThreads)
+struct InfRows {                 // what a row with infinities is multiplied with (affine), and where its products go
+    QMat w;
+    int bits, lg_group, n_out;
+    __nv_bfloat16* y;
+};
+
+// The products of row s (cols values, infinities but no NaN among them) into y: only the infinities count.  One value at
+// a time, so that the kernel around it keeps its registers.
+__device__ __forceinline__ void inf_row(const __nv_bfloat16* s, int cols, const InfRows& r, __nv_bfloat16* y) {
+    const int lane = threadIdx.x & 31;
+    for (int n = threadIdx.x >> 5; n < r.n_out; n += kPrepThreads / 32) {
+        float acc = 0.f;
+#pragma unroll 1
+        for (int k = lane; k < cols; k += 32) {
+            const float x = __bfloat162float(s[k]);
+            if (!isinf(x)) continue;
+            const int bit = (k & 7) * r.bits;                                 // eight codes are r.bits bytes
+            const uint8_t* p = r.w.w + (size_t)n * packed_row_bytes(cols, r.bits) + (size_t)(k >> 3) * r.bits + (bit >> 3);
+            uint32_t q = *p >> (bit & 7);
+            if ((bit & 7) + r.bits > 8) q |= (uint32_t)p[1] << (8 - (bit & 7));
+            const size_t g = (size_t)n * (cols >> r.lg_group) + (k >> r.lg_group);
+            const float sc = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(r.w.scales)[g]);
+            const float bi = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(r.w.biases)[g]);
+            acc += __fadd_rn(__fmul_rn((float)(q & ((1u << r.bits) - 1u)), sc), bi) * x;
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) y[n] = __float2bfloat16_rn(acc);
+    }
+}
+
+// (six blocks an SM: with the registers of five, 2000 rows 2048 -> 8192 in 6 bits took 121.8 instead of 117.9 us)
+template <bool SCALED>
+__global__ void __launch_bounds__(kPrepThreads, 6)
 prepare_one_kernel(const __nv_bfloat16* __restrict__ src, int m, int cols, __half* __restrict__ dst, const Order16 order,
                    const int obits, int unit_rows, int32_t* __restrict__ offsets, int32_t* __restrict__ ident,
                    WorkUnit* __restrict__ units, int32_t* __restrict__ n_units, int32_t* __restrict__ sched, int sched_ints,
-                   float* __restrict__ psum, float* __restrict__ row_scale) {
+                   float* __restrict__ psum, float* __restrict__ row_scale, const InfRows inf) {
     if ((int)blockIdx.x < m) {
         const size_t r = blockIdx.x;
         const __nv_bfloat16* s = src + r * cols;
         __half* d = dst + r * cols;
         float up0 = 1.f, up1 = 1.f;
-        if (row_scale != nullptr) {
+        if (SCALED) {
             __shared__ uint32_t s_mag[kPrepThreads / 32];
             uint32_t mag = 0;
             for (int i = threadIdx.x; i < cols; i += kPrepThreads) mag = max(mag, (uint32_t)__bfloat16_as_ushort(s[i]) & 0x7fffu);
@@ -59,8 +94,11 @@ prepare_one_kernel(const __nv_bfloat16* __restrict__ src, int m, int cols, __hal
             const int k0 = k / 2, k1 = k - k / 2;                             // two factors in fp32's range
             up0 = __uint_as_float((uint32_t)(127 + k0) << 23);
             up1 = __uint_as_float((uint32_t)(127 + k1) << 23);
+            const bool infs = mag == 0x7f80u;
             if (threadIdx.x == 0)
-                row_scale[r] = __uint_as_float((uint32_t)(127 - k0) << 23) * __uint_as_float((uint32_t)(127 - k1) << 23);
+                row_scale[r] = infs ? __uint_as_float(0x7fc00000u)
+                                    : __uint_as_float((uint32_t)(127 - k0) << 23) * __uint_as_float((uint32_t)(127 - k1) << 23);
+            if (infs) inf_row(s, cols, inf, inf.y + r * inf.n_out);
         }
         if (obits >= 0) {
             for (int b = threadIdx.x; b < cols / 16; b += kPrepThreads) {
@@ -312,10 +350,12 @@ int imx_quantized_matmul_ws(const void* x, int m, const imx_qtensor* w, int n_ou
     for (int i = 0; i < 16; ++i) order.o[i] = (int8_t)o[i];
     const bool tmap_second = path == IMX_PATH_DECODE && decode_tmap_supported(set);
     order.pair_scale_odd = tmap_second ? 0.0625f : 1.f;
-    prepare_one_kernel<<<m + 1, 256, 0, stream>>>((const __nv_bfloat16*)x, m, in, ws.x16, order, prep_order(x, order), unit_rows_for(path), ws.offsets,
-                                                  ws.ident, ws.units, ws.n_units, ws.sw.sched, ws.sw.n_ints,
-                                                  tmap_second ? ws.psum : nullptr,
-                                                  path == kPathTwoTerm ? ws.row_scale : nullptr); IMX_LAUNCHED();
+    const bool scaled = path == kPathTwoTerm;
+    const InfRows inf = {set.down, f.bits, f.group == 32 ? 5 : (f.group == 64 ? 6 : 7), n_out, (__nv_bfloat16*)y};
+    auto prepare = scaled ? prepare_one_kernel<true> : prepare_one_kernel<false>;
+    prepare<<<m + 1, kPrepThreads, 0, stream>>>((const __nv_bfloat16*)x, m, in, ws.x16, order, prep_order(x, order), unit_rows_for(path),
+                                                ws.offsets, ws.ident, ws.units, ws.n_units, ws.sw.sched, ws.sw.n_ints,
+                                                tmap_second ? ws.psum : nullptr, ws.row_scale, inf); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     GroupedArgs ga = {};
     ga.set = set;
@@ -330,7 +370,7 @@ int imx_quantized_matmul_ws(const void* x, int m, const imx_qtensor* w, int n_ou
     ga.act = ws.x16;                 // the second product reads its activations here
     ga.act_stride = in;
     ga.out_bf16 = (__nv_bfloat16*)y;
-    ga.row_scale = path == kPathTwoTerm ? ws.row_scale : nullptr;
+    ga.row_scale = scaled ? ws.row_scale : nullptr;
     ga.status = ws.status;
     return run_experts(path, ga, stream);
 }
@@ -367,9 +407,9 @@ int imx_expert_forward(const imx_moe_config* cfg, const imx_qtensor* gate_up, co
     for (int i = 0; i < 16; ++i) order.o[i] = (int8_t)o[i];
     const bool tmap = path == IMX_PATH_DECODE && decode_tmap_supported(set);
     order.pair_scale_odd = tmap ? 0.0625f : 1.f;
-    prepare_one_kernel<<<m + 1, 256, 0, stream>>>((const __nv_bfloat16*)x, m, c.hidden, ws.x16, order, prep_order(x, order), unit_rows_for(path),
-                                                  ws.offsets, ws.ident, ws.units, ws.n_units, ws.sw.sched, ws.sw.n_ints,
-                                                  nullptr, nullptr); IMX_LAUNCHED();
+    prepare_one_kernel<false><<<m + 1, kPrepThreads, 0, stream>>>((const __nv_bfloat16*)x, m, c.hidden, ws.x16, order, prep_order(x, order),
+                                                                  unit_rows_for(path), ws.offsets, ws.ident, ws.units, ws.n_units,
+                                                                  ws.sw.sched, ws.sw.n_ints, nullptr, nullptr, InfRows{}); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     const bool rows_f16 = is_prefill(path);
     GroupedArgs ga = {};

@@ -187,6 +187,11 @@ __device__ __forceinline__ float silu_fast(float g) {
 __device__ __forceinline__ void st_global_u16(void* p, uint32_t v) {
     asm volatile("st.global.u16 [%0], %1;" ::"l"(p), "h"((uint16_t)v) : "memory");
 }
+__device__ __forceinline__ uint16_t ld_global_u16(const void* p) {
+    uint16_t v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ __half2 bf16_to_half2(uint32_t b) {
@@ -945,11 +950,13 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                     // the arithmetic first, for all 32 values and without a branch, then the stores under their
                     // row guards
                     float o[32];
+                    uint32_t written = 0;                           // slots whose rows were written before this launch (BF16)
                     if (a.row_scale != nullptr) {
                         // a weight per slot: one per lane, handed round by shuffle
                         const int my = c * 32 + lane;
                         // (the weight row's own factor, rf, belongs to the lane and is not handed round)
                         const float rs = my < t.rows ? a.row_scale[t.slot0 + my] : 1.f;
+                        if (BF16) written = __ballot_sync(0xffffffffu, rs != rs);
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
                             o[i] = (AFFINE && !TWO ? __uint_as_float(v[i]) : __uint_as_float(v[i]) * rf[0]) * __shfl_sync(0xffffffffu, rs, i);
@@ -961,12 +968,24 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                     const int n_ok = t.rows - c * 32;
                     // (wide tiles: 16-bit rows without a weight per slot went out above)
                     if constexpr (BF16) {
+                        __nv_bfloat16* y = a.out_bf16 + o0;
+                        uint16_t kept[32];                          // (touched only where a row was written before)
+                        if (written != 0)
+                            for (uint32_t w = written; w != 0; w &= w - 1) {
+                                const int i = __ffs(w) - 1;
+                                kept[i] = ld_global_u16(y + (size_t)i * a.set.n_in);
+                            }
 #pragma unroll
                         for (int i = 0; i < 32; i += 2) {
                             const uint32_t h = pack_bf16(o[i], o[i + 1]);
-                            if (i < n_ok) st_global_u16(a.out_bf16 + o0 + (size_t)i * a.set.n_in, h);
-                            if (i + 1 < n_ok) st_global_u16(a.out_bf16 + o0 + (size_t)(i + 1) * a.set.n_in, h >> 16);
+                            if (i < n_ok) st_global_u16(y + (size_t)i * a.set.n_in, h);
+                            if (i + 1 < n_ok) st_global_u16(y + (size_t)(i + 1) * a.set.n_in, h >> 16);
                         }
+                        if (written != 0)
+                            for (uint32_t w = written; w != 0; w &= w - 1) {
+                                const int i = __ffs(w) - 1;
+                                st_global_u16(y + (size_t)i * a.set.n_in, kept[i]);
+                            }
                     } else if (!WIDE && a.out16 != nullptr && a.out_index != nullptr) {
                         // rows scattered to the positions the caller names (expert parallelism: straight into the
                         // buffer the rows travel back in): one index per lane, handed round by shuffle

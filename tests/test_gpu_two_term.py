@@ -1,10 +1,12 @@
 """The tensor-core kernels with two-term weights (affine 3/5/6-bit, 4-bit in groups of 32): the formats whose
 weights stay in 32 bits, against fp64 and against the scalar kernels they replace."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
-from ironmlx_b200 import nn, ops
+from ironmlx_b200 import _lib, nn, ops
 from ironmlx_b200.workloads import MoEConfig
 from oracle import moe as O
 from gpu_util import bf16_to_np, moe_to_device, t_bf16
@@ -53,7 +55,7 @@ def test_linear(cuda, bits, group, m, in_dim, out_dim):
     _check(layer.forward_with_stream(x), x, wd, in_dim)
 
 
-@pytest.mark.parametrize("bits,group,in_dim", [(6, 64, 9728), (6, 64, 11008), (3, 64, 8192), (5, 32, 5120), (4, 32, 4096)])
+@pytest.mark.parametrize("bits,group,in_dim", [(6, 64, 9728), (6, 64, 11008), (3, 64, 8192), (5, 32, 5120), (6, 32, 4096)])
 @pytest.mark.parametrize("m,out_dim", [(3, 384), (20, 512)])
 def test_linear_of_long_rows(cuda, bits, group, in_dim, m, out_dim):
     """Rows of scales that leave little shared memory beside them, with weight tiles that pair up (512) and do not (384)."""
@@ -71,6 +73,33 @@ def test_linear_outside_the_range_of_fp16(cuda, bits, group, x_scale, w_scale):
     x[4] *= 1e-6
     x = x.to(torch.bfloat16)
     _check(layer.forward_with_stream(x), x, wd, 512)
+
+
+@pytest.mark.parametrize("bits,group,m", [(6, 64, 40), (3, 128, 3), (5, 64, 300), (6, 32, 17)])
+def test_linear_rows_with_infinities(cuda, bits, group, m):
+    """Rows with infinities or NaNs come out as the scalar kernel gives them, and leave their neighbours alone."""
+    layer, wd, gen = _layer(cuda, 256, 1024, bits, group, 15)
+    x = torch.randn(m, 1024, generator=gen, device=cuda).to(torch.bfloat16)
+    clean = layer.forward_with_stream(x)
+    inf = float("inf")
+    bad = x.clone()
+    bad[0, 5] = inf
+    bad[1, 700] = -inf
+    bad[1, 1023] = -inf
+    bad[1, 2] = 3e38
+    if m > 3:
+        bad[m - 1, ::7] = inf
+        bad[4, 9], bad[4, 10] = inf, -inf
+        bad[6, 100], bad[6, 101] = inf, float("nan")
+    y = layer.forward_with_stream(bad)
+    want = torch.empty_like(y)
+    qt = layer.qtensor()
+    _lib.check(_lib.lib().imx_quantized_matmul(bad.data_ptr(), m, C.byref(qt), 256, 1024, 1, group, bits, 0, want.data_ptr(),
+                                               torch.cuda.current_stream().cuda_stream))
+    rows = (~torch.isfinite(bad).all(-1)).nonzero()[:, 0]
+    assert torch.isinf(want[0]).any() and torch.equal(torch.nan_to_num(y[rows], nan=5.0), torch.nan_to_num(want[rows], nan=5.0))
+    fine = torch.isfinite(bad).all(-1)
+    assert torch.equal(y[fine], clean[fine])
 
 
 @pytest.mark.parametrize("bits,group", FORMATS)
