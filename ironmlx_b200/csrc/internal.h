@@ -66,6 +66,7 @@ struct RouteScratch {
     const float* inv_rms; // [n] per-token RMSNorm factor: the tiles of x are normalised as they are loaded (or nullptr)
     const void* ln_weight;// bf16 [H] RMSNorm weight that goes with inv_rms (or nullptr)
     const struct RouteSort* sort;   // the dispatch sort is wanted in the router's last launch (or nullptr)
+    int32_t* arrivals;    // word the first launch clears for the second (set by launch_route; or nullptr)
 };
 // Outputs of the dispatch sort done by the router: the CTA that finishes last sorts all assignments.
 struct RouteSort {
@@ -74,7 +75,7 @@ struct RouteSort {
     int32_t* offsets;
     int32_t* perm;
     int32_t* inv_perm;
-    int32_t* arrivals;    // one zeroed word, left zero
+    int32_t* arrivals;    // a word of scratch
 };
 constexpr int kRouteSplitMaxTokens = 1024;   // the split-K router serves batches below this
 int route_slice(int H);                      // K slice of the split-K router (0: not applicable)

@@ -161,6 +161,8 @@ route_splitk_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, co
     const int eb = blockIdx.x, split = blockIdx.y, tb = blockIdx.z;
     const int n_pad = gridDim.z * 32;
     const int tok0 = tb * 32, k0 = split * ks;
+    // whatever a caller's workspace holds there: the next launch counts its CTAs in this word
+    if (rs.arrivals != nullptr && tid == 0 && (eb | split | tb) == 0) *rs.arrivals = 0;
 
     const int cpr = ks >> 3;                                                         // 16-byte pieces per row
     for (int c = tid; c < 32 * cpr; c += kSkThreads) {
@@ -329,7 +331,6 @@ route_finish_kernel(int n_tokens, int n_pad, int n_splits, const float* __restri
         __syncthreads();
         if (!s_last) return;
         __threadfence();
-        if (threadIdx.x == 0) *arrivals = 0;
         SortAux rest = aux;
         rest.sched = nullptr;
         sort_small_block<kFinThreads>(topk_idx, n_tokens * k, E, counts, offsets, perm, inv_perm, rest, reinterpret_cast<int*>(smem_raw));
@@ -363,12 +364,14 @@ int launch_route(const void* x, int n, int H, const void* Wr, const float* logit
     if (rs != nullptr && rs->partials != nullptr && n < kRouteSplitMaxTokens && ks > 0 && E % 32 == 0 && x16 != nullptr) {
         const size_t tiles = (size_t)2 * 32 * (ks + 8) * sizeof(__nv_bfloat16);
         const dim3 grid((unsigned)(E / 32), (unsigned)(H / ks), (unsigned)ceil_div(n, 32));
-        route_splitk_kernel<<<grid, kSkThreads, tiles, stream>>>(
-            (const __nv_bfloat16*)x, n, H, (const __nv_bfloat16*)Wr, logit_bias, E, k, norm, (const __nv_bfloat16*)w_sg,
-            topk_idx, topk_w, shared_gate, (__half*)x16, order, ks, *rs); IMX_LAUNCHED();
-        IMX_CHECK_CUDA(cudaGetLastError());
         const bool sorts = rs->sort != nullptr && sort_done != nullptr && n <= kRouteSortTokens && E <= kSmallSortExperts &&
                            n * k <= kSmallSortIters * kFinThreadsSort;
+        RouteScratch first = *rs;
+        first.arrivals = sorts ? rs->sort->arrivals : nullptr;
+        route_splitk_kernel<<<grid, kSkThreads, tiles, stream>>>(
+            (const __nv_bfloat16*)x, n, H, (const __nv_bfloat16*)Wr, logit_bias, E, k, norm, (const __nv_bfloat16*)w_sg,
+            topk_idx, topk_w, shared_gate, (__half*)x16, order, ks, first); IMX_LAUNCHED();
+        IMX_CHECK_CUDA(cudaGetLastError());
         if (sorts) {
             const RouteSort& so = *rs->sort;
             const size_t ints = std::max((size_t)(kFinThreadsSort / 32) * E, small_sort_ints(kFinThreadsSort / 32, E));

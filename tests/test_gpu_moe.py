@@ -146,6 +146,24 @@ def test_reruns_are_bit_identical(cuda):
     assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
 
 
+@pytest.mark.parametrize("word", [1, 7, -1])
+@pytest.mark.parametrize("tokens", [5, 19])
+def test_small_batches_do_not_rely_on_words_an_earlier_call_left(cuda, tokens, word):
+    """The last CTA of the decode-size router sorts; it is found by a count in the workspace's status block, whatever
+    value that word held before the call."""
+    cfg = MoEConfig("arrivals", tokens=tokens, hidden=512, num_experts=32, top_k=4, intermediate=128, shared_intermediate=128, seed=23)
+    x, p = make_params(cfg)
+    xd = t_bf16(x, cuda)
+    want = moe_to_device(p, cuda).forward_with_stream(xd).clone()
+    moe = moe_to_device(p, cuda)
+    moe.forward_with_stream(xd.flip(0).contiguous())               # leaves the sort of other tokens behind
+    moe._workspace[:64].view(torch.int32)[12] = word
+    y, tr = moe.forward_with_stream(xd, trace=True)
+    assert torch.equal(y, want)
+    assert int(tr["offsets"][-1]) == tokens * cfg.top_k
+    moe.check_status()
+
+
 def test_host_io_entry_point(cuda):
     x, p = make_params(SMALL)
     moe = moe_to_device(p, cuda)
