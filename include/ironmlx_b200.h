@@ -187,7 +187,8 @@ IMX_API int imx_moe_saturations(void* workspace, void* stream, long long* count)
 /* Router (moe.rs:67-82): logits = x.W_r^T (+bias), fp32 softmax, top-k in
  * descending order (lower expert id first among equal values), optional
  * renormalisation; also the shared-expert gate sigmoid(x.w_sg) (moe.rs:174-177)
- * when w_sg != NULL, and an fp16 copy of x for the expert products. */
+ * when w_sg != NULL, and an fp16 copy of x for the expert products.  Should a bounded wait of the kernel
+ * run out, the tokens concerned get experts 0 .. top_k-1 with NaN weights. */
 IMX_API int imx_moe_route(const void* x, int n_tokens, int hidden, const void* router_w,
                   const float* logit_bias, int num_experts, int top_k, int norm_topk_prob,
                   const void* shared_gate_w, int32_t* topk_idx, float* topk_w,

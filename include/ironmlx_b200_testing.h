@@ -21,4 +21,12 @@ extern "C"
 #endif
 __attribute__((visibility("default"))) void imx_testing_decode_handoff(int spin_limit, int withhold);
 
+/* With on != 0 every wait of the router of larger batches gives up before its first try, so that nothing is copied or
+ * multiplied: its tokens get experts 0 .. k-1 with NaN weights, and status 3 is recorded where the caller has a status
+ * word.  0 restores the default.  Process-wide. */
+#ifdef __cplusplus
+extern "C"
+#endif
+__attribute__((visibility("default"))) void imx_testing_route_give_up(int on);
+
 #endif /* IRONMLX_B200_TESTING_H */

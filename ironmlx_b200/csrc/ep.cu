@@ -403,7 +403,7 @@ int forward_gathered(imx_ep_ctx& x, const imx_moe_weights* w, const void* xin, i
     bool sums_done = false;
     IMX_TRY(launch_route(ws.xg, nA, c.hidden, w->router_w, w->router_logit_bias, c.num_experts, c.top_k, c.norm_topk_prob,
                          has_shared ? w->shared_expert_gate_w : nullptr, ws.topk_idx, ws.topk_w, ws.shared_gate, ws.x16, order,
-                         stream, tmap_decode ? 0.0625f : 1.f, ws.route_partials ? &rs : nullptr, &sums_done));
+                         stream, tmap_decode ? 0.0625f : 1.f, ws.route_partials ? &rs : nullptr, &sums_done, ws.c.status));
     const int nmax = A > n ? A : n;
     local_ids_kernel<<<(nmax + 255) / 256, 256, 0, stream>>>(ws.topk_idx, A, x.rank * x.e_loc, ws.ids_local, ws.ident, n); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
@@ -505,7 +505,7 @@ int forward_a2a(imx_ep_ctx& x, const imx_moe_weights* w, const void* xin, int n,
     RouteScratch rs = {ws.route_partials, ws.route_sg, nullptr, nullptr, nullptr};
     IMX_TRY(launch_route(xin, n, H, w->router_w, w->router_logit_bias, E, c.top_k, c.norm_topk_prob,
                          has_shared ? w->shared_expert_gate_w : nullptr, ws.topk_idx, ws.topk_w, ws.shared_gate, x16, order,
-                         stream, 1.f, ws.route_partials ? &rs : nullptr, nullptr));
+                         stream, 1.f, ws.route_partials ? &rs : nullptr, nullptr, ws.c.status));
     // 2. stable sort by global expert id, rows packed in that order
     SortExtras ex;
     ex.topk_w = ws.topk_w;

@@ -11,7 +11,11 @@
 //
 // Sixteen warps: 0 issues the MMAs, 1 owns tensor memory, 2 loads, 4..7 move the logits (lane = expert, column =
 // token) into shared memory, 8..15 write the fp16 copy and the gate while the product runs; then all take tokens'
-// softmax and top-k.  Every wait is bounded; on expiry the status word is set and tensor memory freed.
+// softmax and top-k.  Every wait is bounded.  On expiry the CTA waits for its copies and MMAs in flight, frees tensor
+// memory, sets the caller's status word where there is one, and gives its tokens experts 0 .. k-1 (valid, whatever is done
+// with them next) with NaN weights, which no result can hide.
+#include <atomic>
+
 #include "route_common.cuh"
 #include "tcgen05.cuh"
 
@@ -27,11 +31,13 @@ constexpr int kRtK = 64;
 constexpr int kRtMaxStages = 6;
 constexpr int kRtMaxExperts = 256;
 constexpr size_t kRtSmemMost = 227 * 1024;
+std::atomic<int> g_route_spin_limit{kSpin};
 
 struct RtBars {
     uint64_t full[kRtMaxStages];
     uint64_t empty[kRtMaxStages];
     uint64_t acc_full;
+    uint64_t retired;                              // after an expired wait: the MMAs issued before it
     uint32_t tmem_base;
     int abort;
 };
@@ -45,7 +51,7 @@ __global__ void __launch_bounds__(kRtThreads, 1)
 route_tc_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, int E, const float* __restrict__ logit_bias, int k,
                 int norm, const __nv_bfloat16* __restrict__ w_sg, int32_t* __restrict__ topk_idx, float* __restrict__ topk_w,
                 float* __restrict__ shared_gate, __half* __restrict__ x16, const int obits, const float pair_scale_odd,
-                const int stages, int32_t* __restrict__ status, const __grid_constant__ RtMaps maps) {
+                const int stages, const int spin_limit, int32_t* __restrict__ status, const __grid_constant__ RtMaps maps) {
     constexpr uint32_t kTmem = 2 * NTOK;                     // columns: two accumulators of NTOK
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -66,6 +72,7 @@ route_tc_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, int E,
             mbar_init(smem_u32(&bars->empty[s]), 1);
         }
         mbar_init(smem_u32(&bars->acc_full), 1);
+        mbar_init(smem_u32(&bars->retired), 1);
         bars->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -79,6 +86,7 @@ route_tc_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, int E,
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
+    int copied = 0;                                          // K steps the loader has started
 
     if (warp == 0) {
         int s = 0;
@@ -86,7 +94,7 @@ route_tc_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, int E,
         // bf16 x bf16 -> fp32
         const uint32_t idesc = idesc_for(128, NTOK) | (1u << 7) | (1u << 10);
         for (int ks = 0; ks < ksteps; ++ks) {
-            if (!mbar_wait(smem_u32(&bars->full[s]), ph, abort_flag)) break;
+            if (!mbar_wait(smem_u32(&bars->full[s]), ph, abort_flag, spin_limit)) break;
             tc_fence_after();
             if (elect_one()) {
                 const uint32_t stage = sbase + (uint32_t)s * stage_bytes;
@@ -107,8 +115,8 @@ route_tc_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, int E,
     } else if (warp == 2) {
         int s = 0;
         uint32_t ph = 0;
-        for (int ks = 0; ks < ksteps; ++ks) {
-            if (!mbar_wait(smem_u32(&bars->empty[s]), ph ^ 1u, abort_flag)) break;
+        for (int ks = 0; ks < ksteps; ++ks, ++copied) {
+            if (!mbar_wait(smem_u32(&bars->empty[s]), ph ^ 1u, abort_flag, spin_limit)) break;
             if (lane == 0) {
                 const uint32_t stage = sbase + (uint32_t)s * stage_bytes, bar = smem_u32(&bars->full[s]);
                 mbar_expect_tx(bar, stage_bytes);
@@ -122,7 +130,7 @@ route_tc_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, int E,
             }
         }
     } else if (warp >= 4 && warp < 8) {
-        if (mbar_wait(smem_u32(&bars->acc_full), 0u, abort_flag)) {
+        if (mbar_wait(smem_u32(&bars->acc_full), 0u, abort_flag, spin_limit)) {
             tc_fence_after();
             const int q = warp & 3;
             for (int h = 0; h < halves; ++h) {
@@ -170,9 +178,26 @@ route_tc_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, int E,
         }
     }
     __syncthreads();
+    const bool gave_up = bars->abort != 0;
+    if (gave_up) {
+        if (warp == 0) {
+            if (elect_one()) umma_commit(smem_u32(&bars->retired));
+            __syncwarp();
+            mbar_drain(smem_u32(&bars->retired), 0u);
+        } else if (warp == 2) {
+            for (int ks = max(0, copied - stages); ks < copied; ++ks)
+                mbar_drain(smem_u32(&bars->full[ks % stages]), (uint32_t)(ks / stages) & 1u);
+        }
+        __syncthreads();
+    }
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmem) : "memory");
-    if (bars->abort) {
+    if (gave_up) {
         if (tid == 0 && status != nullptr) atomicExch(status, 3);
+        const long first = (long)tok0 * k, last = (long)min(n_tokens, tok0 + NTOK) * k;
+        for (long i = first + tid; i < last; i += kRtThreads) {
+            topk_idx[i] = (int32_t)((i - first) % k);
+            topk_w[i] = __uint_as_float(0x7fc00000u);
+        }
         return;
     }
     for (int r = warp; r < NTOK; r += kRtThreads / 32) {
@@ -203,12 +228,15 @@ int launch_tile(const void* x, int n, int H, const void* Wr, const float* logit_
     IMX_TRY(make_tensor_map_2d(Wr, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (size_t)E, (size_t)H, (size_t)H * 2, kRtK, 128, true, &maps.w));
     route_tc_kernel<NTOK><<<ceil_div(n, NTOK), kRtThreads, ring + fixed, stream>>>(
         (const __nv_bfloat16*)x, n, H, E, logit_bias, k, norm, (const __nv_bfloat16*)w_sg, topk_idx, topk_w, shared_gate,
-        (__half*)x16, order_bits(order), order.pair_scale_odd, stages, status, maps); IMX_LAUNCHED();
+        (__half*)x16, order_bits(order), order.pair_scale_odd, stages, g_route_spin_limit.load(), status, maps); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     return IMX_OK;
 }
 
 }  // namespace
+
+// Test hook (include/ironmlx_b200_testing.h).
+void testing_route_give_up(int on) { g_route_spin_limit.store(on ? 0 : kSpin); }
 
 // A tile takes all K steps one after the other whatever the batch (15 us at a hidden size of 512, 29 at 2048, 73 at 9728),
 // the cluster-per-token kernel's time grows with the tokens and, less, with the experts; it serves the batches that this

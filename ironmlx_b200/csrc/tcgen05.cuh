@@ -54,13 +54,17 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Bounded wait; false (and the abort flag set) when it gives up or someone else did.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    for (int spin = 0; spin < kSpin; ++spin) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int limit = kSpin) {
+    for (int spin = 0; spin < limit; ++spin) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((spin & 1023) == 1023 && *abort_flag) return false;
     }
     *abort_flag = 1;
     return false;
+}
+// The wait for what is still in flight once a kernel has given up: bounded too, and nothing follows from it.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+    for (int spin = 0; spin < kSpin && !mbar_try_wait(bar, parity); ++spin) {}
 }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");

@@ -11,6 +11,7 @@ import pytest
 import torch
 
 from ironmlx_b200 import _lib
+from ironmlx_b200.ep import CudaStages
 from ironmlx_b200.workloads import MoEConfig, round_bf16
 from oracle import moe as O
 from gpu_util import bf16_to_np, moe_to_device, t_bf16
@@ -67,6 +68,33 @@ def test_a_clamp_is_counted(cuda, path):
     moe.check_status()
     assert moe.saturations() > 0
     assert moe.saturations() == 0                       # reading clears the count
+
+
+def test_expired_router_wait_is_reported_and_shows_in_the_result(cuda):
+    """The router of larger batches with waits that give up at once: the status word says so, no output is a number, the
+    stage call without a status word returns NaN weights, and the next call is correct."""
+    cfg = MoEConfig("give-up", tokens=1100, hidden=512, num_experts=8, top_k=2, intermediate=128, shared_intermediate=128, seed=94)
+    x, p = make_params(cfg)
+    moe = moe_to_device(p, cuda)
+    xd = t_bf16(x, cuda)
+    good = moe.forward_with_stream(xd).clone()
+    moe.check_status()
+    lib = _lib.lib()
+    stages = CudaStages(cuda)
+    try:
+        lib.imx_testing_route_give_up(1)
+        y = moe.forward_with_stream(xd)
+        with pytest.raises(_lib.IronMLXError) as e:
+            moe.check_status()
+        assert e.value.code == _lib.ERR_DEVICE and "status 3" in str(e.value)
+        assert torch.isnan(y).all()
+        idx, w, _, _ = stages.route(xd, moe.gate.weight, None, 2, True, None)
+        assert torch.isnan(w).all() and torch.equal(idx, torch.arange(2, device=cuda, dtype=torch.int32).expand(1100, 2))
+    finally:
+        lib.imx_testing_route_give_up(0)
+    again = moe.forward_with_stream(xd)
+    moe.check_status()
+    assert torch.equal(again, good)
 
 
 def test_expired_handoff_wait_is_reported_and_the_gpu_stays_usable(cuda):
