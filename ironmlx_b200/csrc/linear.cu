@@ -37,6 +37,7 @@ namespace {
 // meet weights split into two terms, inf * hi + inf * lo, which is NaN wherever the signs differ: its products, infinities
 // by the sign of the weights that meet one (NaN for a zero or opposite ones), are written here, and a NaN for its factor
 // tells the product's epilogue to leave them.
+// SAT: values beyond fp16's range are clamped, as in the block (SwiGLU admits no factor per row).
 constexpr int kPrepThreads = 256;
 
 struct InfRows {                 // what a row with infinities is multiplied with (affine), and where its products go
@@ -70,7 +71,7 @@ __device__ __forceinline__ void inf_row(const __nv_bfloat16* s, int cols, const 
 }
 
 // (six blocks an SM: with the registers of five, 2000 rows 2048 -> 8192 in 6 bits took 121.8 instead of 117.9 us)
-template <bool SCALED>
+template <bool SCALED, bool SAT>
 __global__ void __launch_bounds__(kPrepThreads, 6)
 prepare_one_kernel(const __nv_bfloat16* __restrict__ src, int m, int cols, __half* __restrict__ dst, const Order16 order,
                    const int obits, int unit_rows, int32_t* __restrict__ offsets, int32_t* __restrict__ ident,
@@ -102,7 +103,7 @@ prepare_one_kernel(const __nv_bfloat16* __restrict__ src, int m, int cols, __hal
         }
         if (obits >= 0) {
             for (int b = threadIdx.x; b < cols / 16; b += kPrepThreads) {
-                const float sum = route::convert_block16<false>(obits, s + b * 16, d + b * 16, order.pair_scale_odd, up0, up1);
+                const float sum = route::convert_block16<SAT>(obits, s + b * 16, d + b * 16, order.pair_scale_odd, up0, up1);
                 if (psum != nullptr) psum[r * (cols / 16) + b] = sum;
             }
             return;
@@ -112,7 +113,8 @@ prepare_one_kernel(const __nv_bfloat16* __restrict__ src, int m, int cols, __hal
             float sum = 0.f;
             for (int i = 0; i < 16; ++i) {
                 const float v = __bfloat162float(s[b * 16 + order.o[i]]) * up0 * up1;
-                const __half h = __float2half_rn((i & 2) ? v * order.pair_scale_odd : v);
+                const float u = (i & 2) ? v * order.pair_scale_odd : v;
+                const __half h = SAT ? f32_to_f16_sat(u) : __float2half_rn(u);
                 d[b * 16 + i] = h;
                 sum += (i & 2) ? __half2float(h) * (1.f / order.pair_scale_odd) : __half2float(h);
             }
@@ -352,7 +354,7 @@ int imx_quantized_matmul_ws(const void* x, int m, const imx_qtensor* w, int n_ou
     order.pair_scale_odd = tmap_second ? 0.0625f : 1.f;
     const bool scaled = path == kPathTwoTerm;
     const InfRows inf = {set.down, f.bits, f.group == 32 ? 5 : (f.group == 64 ? 6 : 7), n_out, (__nv_bfloat16*)y};
-    auto prepare = scaled ? prepare_one_kernel<true> : prepare_one_kernel<false>;
+    auto prepare = scaled ? prepare_one_kernel<true, false> : prepare_one_kernel<false, false>;
     prepare<<<m + 1, kPrepThreads, 0, stream>>>((const __nv_bfloat16*)x, m, in, ws.x16, order, prep_order(x, order), unit_rows_for(path),
                                                 ws.offsets, ws.ident, ws.units, ws.n_units, ws.sw.sched, ws.sw.n_ints,
                                                 tmap_second ? ws.psum : nullptr, ws.row_scale, inf); IMX_LAUNCHED();
@@ -407,9 +409,13 @@ int imx_expert_forward(const imx_moe_config* cfg, const imx_qtensor* gate_up, co
     for (int i = 0; i < 16; ++i) order.o[i] = (int8_t)o[i];
     const bool tmap = path == IMX_PATH_DECODE && decode_tmap_supported(set);
     order.pair_scale_odd = tmap ? 0.0625f : 1.f;
-    prepare_one_kernel<false><<<m + 1, kPrepThreads, 0, stream>>>((const __nv_bfloat16*)x, m, c.hidden, ws.x16, order, prep_order(x, order),
-                                                                  unit_rows_for(path), ws.offsets, ws.ident, ws.units, ws.n_units,
-                                                                  ws.sw.sched, ws.sw.n_ints, nullptr, nullptr, InfRows{}); IMX_LAUNCHED();
+    // an infinity in fp16 is NaN after two terms, or after an MMA that meets a zero weight, and takes the whole row along
+    // with it; the decode and scalar kernels clamp what follows from it to fp16's range instead
+    const bool sat = path == kPathTwoTerm || path == kPathTcRows32;
+    auto prepare = sat ? prepare_one_kernel<false, true> : prepare_one_kernel<false, false>;
+    prepare<<<m + 1, kPrepThreads, 0, stream>>>((const __nv_bfloat16*)x, m, c.hidden, ws.x16, order, prep_order(x, order),
+                                                unit_rows_for(path), ws.offsets, ws.ident, ws.units, ws.n_units,
+                                                ws.sw.sched, ws.sw.n_ints, nullptr, nullptr, InfRows{}); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     const bool rows_f16 = is_prefill(path);
     GroupedArgs ga = {};

@@ -114,3 +114,25 @@ def test_quantized_linear_into_rows_at_any_value(cuda, mode, bits, group, m, at)
         assert torch.equal(got, want)
     assert lib.imx_quantized_matmul_ws(x.data_ptr(), m, C.byref(qt), n_out, n_in, *fmt, buf.data_ptr() + 1,
                                        scratch.data_ptr(), nb.value, torch.cuda.current_stream().cuda_stream) == _lib.ERR_INVALID
+
+
+@pytest.mark.parametrize("mode,bits,group,m", [("affine", 6, 64, 3), ("affine", 3, 64, 70), ("mxfp8", 8, 32, 12), ("nvfp4", 4, 16, 20)])
+def test_expert_rows_beyond_the_range_of_fp16(cuda, mode, bits, group, m):
+    """The fp16 copy of an expert's input is clamped to +-65504, as in the block: the outputs are those of the clamped
+    rows (fp16 carries them exactly), and rows beside them are not touched."""
+    from gpu_util import moe_to_device
+    from util import make_params
+    cfg = MoEConfig("range", m, 1024, 1, 1, 512, 0, mode=mode, bits=bits, group_size=group, seed=31)
+    x, p = make_params(cfg)
+    expert = moe_to_device(p, cuda)._fused.expert(0)
+    xd = t_bf16(x, cuda)
+    clean = expert.forward_with_stream(xd)
+    xd[1, 7], xd[1, 100] = 1e5, -float("inf")
+    y = expert.forward_with_stream(xd)
+    clamped = bf16_to_np(xd[1:2]).clip(-65504.0, 65504.0).astype(np.float64)
+    wg, wu, wd = (w.astype(np.float64) for w in O.expert_weights(p, 0))
+    with np.errstate(over="ignore"):
+        act = np.clip(O.silu(clamped @ wg.T) * (clamped @ wu.T), -65504.0, 65504.0)
+    assert O.rel_l2(bf16_to_np(y[1:2]), act @ wd.T) <= TOL
+    rest = torch.arange(m, device=cuda) != 1
+    assert torch.equal(y[rest], clean[rest])
