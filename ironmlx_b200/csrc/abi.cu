@@ -181,18 +181,32 @@ bool is_decode(int path) { return path == IMX_PATH_DECODE || path == IMX_PATH_DE
 bool decode_supported(const ExpertSet& s) { return decode_mma_supported(s) || decode_fp_supported(s); }
 
 // Between decode and prefill sizes the decode kernels take an expert's rows through its weights eight at a time, the
-// tensor-core kernels 256 at a time; both keep rows in fp32 and weights exact (block-scaled floats) or in 32 bits
-// (two-term).  Rows an expert (on average) from which the latter are faster, measured on a B200 as us a block:
-//   mxfp8  8   (256 experts of 2048 x 512: 4 rows 310 / 310, 8 rows 425 / 320, 28 rows 1093 / 362; 64 of 1024 x 512: 4 rows 77 / 89)
-//   nvfp4  16  (8 rows 239 / 306, 16 rows 384 / 319, 28 rows 591 / 343)
-static long rows32_from(const ExpertSet& s) { return (s.fmt.mode == IMX_MODE_MXFP8 ? 8L : 16L) * s.num_experts; }
-//   affine, register-pipelined decode kernel  16  (8-bit: 8 rows 400 / 509, 16 rows 671 / 519, 28 rows 1080 / 557; 2-bit:
-//          16 rows 546 / 468), and 128 where the weight tiles do not fill the GPU (16 experts of 512 x 256: 64 rows
-//          62.5 / 70.4, 128 rows 76.8 / 72.7, 256 rows 112 / 79)
+// tensor-core kernels 256 at a time.  Both keep rows in fp32; the latter take block-scaled floats exactly and affine weights
+// as two fp16 terms (22 bits, see TwoTerm).  From how many rows an expert (on average) they are faster depends on how many
+// of their weight tiles (64 columns of an expert) there are for an SM: a few tiles are bound by their start and end.
+// Measured on a B200, us a block, decode / tensor-core:
+//   many tiles, 256 experts of 2048 x 512 (14 an SM): mxfp8 8 rows 397 / 317; nvfp4 8 rows 239 / 306, 16 rows 379 / 317;
+//     8-bit 8 rows 400 / 509, 16 rows 662 / 513; 2-bit 16 rows 538 / 464
+//   64 of 1024 x 512 and 128 of 1024 x 256 (3.5 an SM): mxfp8 8 rows 92 / 88; nvfp4 16 rows 79 / 87, 20 rows 90 / 88; 8-bit
+//     16 rows 106 / 126, 20 rows 132 / 126; 2-bit 16 rows 106 / 108, 20 rows 122 / 107; 4-bit 20 rows 113 / 117, 24 rows 124 / 121
+//   8 of 2048 x 1024 (0.9 an SM): mxfp8 8 rows 72 / 55; nvfp4 16 rows 52 / 54, 24 rows 57 / 55
+//   16 of 512 x 256 (0.4 an SM): mxfp8 31 rows 40 / 42, 64 rows 44 / 46, 100 rows 62 / 53; nvfp4 31 rows 33 / 41, 128 rows
+//     51 / 49; 8-bit 128 rows 62 / 59; one expert of 2048 x 512: mxfp8 8 rows 49 / 35, nvfp4 31 rows 31 / 35
 //   affine 4-bit in groups of 64, tensor-map decode kernel: not below prefill sizes (28 rows 486 / 546)
+static bool tiles_per_sm(const ExpertSet& s, double at_least) {
+    DeviceInfo di;
+    const int sms = current_device(&di) == IMX_OK ? di.sms : 148;
+    return (double)s.num_experts * s.n_mid / 64 >= at_least * sms;
+}
+static long rows32_from(const ExpertSet& s) {
+    const bool few = !tiles_per_sm(s, 0.5);
+    if (s.fmt.mode == IMX_MODE_MXFP8) return (few && s.num_experts > 1 ? 96L : 8L) * s.num_experts;
+    return (few ? 128L : (tiles_per_sm(s, 8) ? 16L : 20L)) * s.num_experts;
+}
 static long two_term_from(const ExpertSet& s) {
     if (decode_tmap_supported(s)) return 1L << 40;
-    return ((long)s.num_experts * s.n_mid / 128 >= 148 ? 16L : 128L) * s.num_experts;
+    if (!tiles_per_sm(s, 2)) return 128L * s.num_experts;
+    return (tiles_per_sm(s, 8) ? 16L : (s.fmt.bits == 4 ? 24L : 20L)) * s.num_experts;
 }
 // Which expert kernels run for this call.  AUTO: tensor-memory GEMM tiles once
 // experts see enough rows to fill them, the decode kernels below that.
