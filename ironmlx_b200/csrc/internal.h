@@ -195,7 +195,7 @@ unsigned long long launch_count();   // kernels this library has launched (or re
 // One-time set-up per (device, kernel family): attributes such as the dynamic shared-memory limit are per
 // device, so a process that drives several GPUs sets them on each.  The first call on a device should come
 // before any stream capture.
-enum { kSetupDecodeTmap = 0, kSetupPrefillTc = 1, kSetupRouteTc = 2 };
+enum { kSetupDecodeTmap = 0, kSetupRouteTc = 1, kSetupPrefillTc = 2 /* + the weight format: 11 of them */ };
 bool device_needs_setup(int ordinal, int family);
 void device_mark_setup(int ordinal, int family);
 // Tiled TMA descriptor of a 2-D row-major matrix [rows, cols] of `esize`-byte elements, `ld_bytes` between

@@ -1253,8 +1253,13 @@ struct Plan {
 };
 
 template <int FMT>
-int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, const TcMaps& mgu, const TcMaps& mdn, int sms,
-               cudaStream_t stream, cudaEvent_t mid) {
+int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, const TcMaps& mgu, const TcMaps& mdn, const DeviceInfo& di,
+               bool first, cudaStream_t stream, cudaEvent_t mid) {
+    const int sms = di.sms;
+    if (first) {
+        IMX_TRY(configure<FMT>());
+        device_mark_setup(di.ordinal, kSetupPrefillTc + FMT);
+    }
     if (a.out_bf16 != nullptr) {
         if (dn.pair) prefill_pair_kernel<false, FMT, true><<<sms & ~1, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
         else if (dn.wide) prefill_tc_kernel<false, FMT, true, true, false, true><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
@@ -1410,21 +1415,6 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
 
     DeviceInfo di;
     IMX_TRY(current_device(&di));
-    if (device_needs_setup(di.ordinal, kSetupPrefillTc)) {   // once per device, outside any stream capture (first call)
-        IMX_TRY(configure<FMT_A4>());
-        IMX_TRY(configure<FMT_A8>());
-        IMX_TRY(configure<FMT_A2>());
-        IMX_TRY(configure<FMT_MXFP8>());
-        IMX_TRY(configure<FMT_NVFP4>());
-        IMX_TRY(configure<FMT_T2>());
-        IMX_TRY(configure<FMT_T3>());
-        IMX_TRY(configure<FMT_T4>());
-        IMX_TRY(configure<FMT_T5>());
-        IMX_TRY(configure<FMT_T6>());
-        IMX_TRY(configure<FMT_T8>());
-        device_mark_setup(di.ordinal, kSetupPrefillTc);
-    }
-
     auto plan = [&](int K_max, int K_min, bool wide, bool xr, Plan* out) -> bool {
         return make_plan(f, fmt, K_max, K_min, wide, xr, ts, out);
     };
@@ -1484,18 +1474,20 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
     }
     mdn.w[2] = mdn.w[1];
 
+    // attributes of the format's kernels, once per device (the first call, outside any stream capture)
+    const bool first = device_needs_setup(di.ordinal, kSetupPrefillTc + fmt);
     switch (fmt) {
-        case FMT_A4: return launch_fmt<FMT_A4>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_A8: return launch_fmt<FMT_A8>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_A2: return launch_fmt<FMT_A2>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_MXFP8: return launch_fmt<FMT_MXFP8>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_NVFP4: return launch_fmt<FMT_NVFP4>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_T2: return launch_fmt<FMT_T2>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_T8: return launch_fmt<FMT_T8>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_T3: return launch_fmt<FMT_T3>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_T4: return launch_fmt<FMT_T4>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_T5: return launch_fmt<FMT_T5>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
-        case FMT_T6: return launch_fmt<FMT_T6>(a, gu, dn, ts, mgu, mdn, di.sms, stream, mid);
+        case FMT_A4: return launch_fmt<FMT_A4>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_A8: return launch_fmt<FMT_A8>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_A2: return launch_fmt<FMT_A2>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_MXFP8: return launch_fmt<FMT_MXFP8>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_NVFP4: return launch_fmt<FMT_NVFP4>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_T2: return launch_fmt<FMT_T2>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_T8: return launch_fmt<FMT_T8>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_T3: return launch_fmt<FMT_T3>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_T4: return launch_fmt<FMT_T4>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_T5: return launch_fmt<FMT_T5>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
+        case FMT_T6: return launch_fmt<FMT_T6>(a, gu, dn, ts, mgu, mdn, di, first, stream, mid);
     }
     set_error("prefill path: unknown format");
     return IMX_ERR_INVALID;
