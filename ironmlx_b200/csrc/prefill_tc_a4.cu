@@ -1,0 +1,5 @@
+#include "prefill_tc.cuh"
+
+namespace imx::prefill {
+IMX_TC_FORMAT(FMT_A4)
+}
