@@ -721,7 +721,9 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             // [lane group of 16][gate, up], or the weight rows 16 gs + 8 r8 + lane / 4 of the warp's 32; second product
             // with one weight row a lane (fp32 rows): [0]
             float rf[4] = {1.f, 1.f, 1.f, 1.f};
-            const bool frag_rows = !SWIGLU && WIDE && p.epi_bytes != 0;
+            // rows that leave through the transposing buffer: the launch planned one (fp16 rows without a weight per slot
+            // always have it; asked of the plan as well, their kernels came out 0.5 % slower)
+            const bool frag_rows = !SWIGLU && WIDE && (BF16 ? p.epi_bytes != 0 : a.row_scale == nullptr && a.out16 != nullptr);
             if (SWIGLU) {
 #pragma unroll
                 for (int gs = 0; gs < 2; ++gs) {
@@ -900,13 +902,13 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                     // the arithmetic first, for all 32 values and without a branch, then the stores under their
                     // row guards
                     float o[32];
-                    uint32_t written = 0;                           // slots whose rows were written before this launch (BF16)
+                    uint32_t written = 0;                           // slots whose rows were written before this launch
                     if (a.row_scale != nullptr) {
                         // a weight per slot: one per lane, handed round by shuffle
                         const int my = c * 32 + lane;
                         // (the weight row's own factor, rf, belongs to the lane and is not handed round)
                         const float rs = my < t.rows ? a.row_scale[t.slot0 + my] : 1.f;
-                        if (BF16) written = __ballot_sync(0xffffffffu, rs != rs);
+                        if (BF16 && TWO) written = __ballot_sync(0xffffffffu, rs != rs);
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
                             o[i] = (AFFINE && !TWO ? __uint_as_float(v[i]) : __uint_as_float(v[i]) * rf[0]) * __shfl_sync(0xffffffffu, rs, i);
@@ -920,7 +922,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                     if constexpr (BF16) {
                         __nv_bfloat16* y = a.out_bf16 + o0;
                         uint16_t kept[32];                          // (touched only where a row was written before)
-                        if (written != 0)
+                        if (TWO && written != 0)
                             for (uint32_t w = written; w != 0; w &= w - 1) {
                                 const int i = __ffs(w) - 1;
                                 kept[i] = ld_global_u16(y + (size_t)i * a.set.n_in);
@@ -931,7 +933,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                             if (i < n_ok) st_global_u16(y + (size_t)i * a.set.n_in, h);
                             if (i + 1 < n_ok) st_global_u16(y + (size_t)(i + 1) * a.set.n_in, h >> 16);
                         }
-                        if (written != 0)
+                        if (TWO && written != 0)
                             for (uint32_t w = written; w != 0; w &= w - 1) {
                                 const int i = __ffs(w) - 1;
                                 st_global_u16(y + (size_t)i * a.set.n_in, kept[i]);
