@@ -29,4 +29,10 @@ extern "C"
 #endif
 __attribute__((visibility("default"))) void imx_testing_route_give_up(int on);
 
+/* The same for the tensor-core expert products: their rows are not written, status 3 is recorded. */
+#ifdef __cplusplus
+extern "C"
+#endif
+__attribute__((visibility("default"))) void imx_testing_prefill_give_up(int on);
+
 #endif /* IRONMLX_B200_TESTING_H */

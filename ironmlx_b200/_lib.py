@@ -69,6 +69,7 @@ SIGNATURES = {
     "imx_moe_status": (_i, [_vp, _vp]),
     "imx_testing_decode_handoff": (None, [_i, _i]),
     "imx_testing_route_give_up": (None, [_i]),
+    "imx_testing_prefill_give_up": (None, [_i]),
     "imx_moe_saturations": (_i, [_vp, _vp, C.POINTER(C.c_longlong)]),
     "imx_moe_route": (_i, [_vp, _i, _i, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp]),
     "imx_moe_route_scratch_bytes": (_i, [_i, _i, _i, C.POINTER(_sz)]),

@@ -540,6 +540,7 @@ int imx_moe_status(void* workspace, void* stream_) {
 
 void imx_testing_decode_handoff(int spin_limit, int withhold) { testing_decode_handoff(spin_limit, withhold); }
 void imx_testing_route_give_up(int on) { testing_route_give_up(on); }
+void imx_testing_prefill_give_up(int on) { testing_prefill_give_up(on); }
 
 int imx_moe_saturations(void* workspace, void* stream_, long long* count) {
     IMX_REQUIRE(workspace != nullptr && count != nullptr, "saturations: workspace and count are required");

@@ -167,6 +167,8 @@ bool decode_tmap_supported(const ExpertSet& s);
 int launch_decode_tmap(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid = nullptr);
 void testing_decode_handoff(int spin_limit, int withhold);
 void testing_route_give_up(int on);
+void testing_prefill_give_up(int on);
+constexpr int kSpin = 1 << 22;               // bound of the waits of the tensor-core kernels
 // Decode kernel of the block-scaled float formats (mxfp8, nvfp4).
 bool decode_fp_supported(const ExpertSet& s);
 int launch_decode_fp(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid = nullptr);

@@ -1,5 +1,6 @@
 // Host side of the tensor-core expert products (prefill_tc.cuh): which shapes and formats they take, the shared-memory plan,
 // tensor maps and the launch.
+#include <atomic>
 #include <cstring>
 
 #include "prefill_tc.h"
@@ -9,6 +10,8 @@ namespace imx {
 using namespace prefill;
 
 namespace {
+
+std::atomic<int> g_spin_limit{kSpin};
 
 int fmt_index(const QFormat& f) {
     if (f.mode == IMX_MODE_AFFINE) return f.bits == 4 ? FMT_A4 : (f.bits == 8 ? FMT_A8 : (f.bits == 2 ? FMT_A2 : -1));
@@ -70,6 +73,7 @@ bool make_plan(const QFormat& f, int fmt, int K_max, int K_min, bool wide, bool 
     out->p.sc_bytes = (int)sc;
     out->p.panel_bytes = (int)panel;
     out->p.epi_bytes = (int)epi;
+    out->p.spin_limit = g_spin_limit.load();
     out->p.lg_group = log2_exact(f.group);
     out->smem = fixed + (size_t)st * stage;
     out->wide = wide;
@@ -100,6 +104,9 @@ int read_prof(unsigned long long* out32);
 }
 extern "C" IMX_API int imx_debug_tc_prof(unsigned long long* out32) { return prefill::read_prof<prefill::FMT_A4>(out32); }
 #endif
+
+// Test hook (include/ironmlx_b200_testing.h).
+void testing_prefill_give_up(int on) { g_spin_limit.store(on ? 0 : kSpin); }
 
 static bool tc_supported(const ExpertSet& s, bool second_only, bool (*ok)(int, const QFormat&)) {
     const QFormat& f = s.fmt;

@@ -551,6 +551,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             mbar_init(smem_u32(&bars->sfull[b]), 1);
             mbar_init(smem_u32(&bars->sempty[b]), 8);
         }
+        mbar_init(smem_u32(&bars->retired), 1);
         bars->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -583,7 +584,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
         for_each_tile<SWIGLU, XR, SPLIT, PAIR>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
             const int buf = it % NB, round = it / NB;
             PROF_BEGIN
-            if (!mbar_wait(smem_u32(&bars->acc_empty[buf]), (uint32_t)(round & 1) ^ 1u, abort_flag)) return false;
+            if (!mbar_wait(smem_u32(&bars->acc_empty[buf]), (uint32_t)(round & 1) ^ 1u, abort_flag, p.spin_limit)) return false;
             PROF_END(0)
             tc_fence_after();
             const int ksteps = t.K / kTileK;
@@ -591,7 +592,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             const uint32_t d = tmem + (uint32_t)(buf * DCOLS);
             for (int ks = 0; ks < ksteps; ++ks) {
                 PROF_BEGIN
-                if (!mbar_wait(smem_u32(&bars->full[r.s]), r.ph, abort_flag)) return false;
+                if (!mbar_wait(smem_u32(&bars->full[r.s]), r.ph, abort_flag, p.spin_limit)) return false;
                 PROF_END(1)
                 tc_fence_after();
                 PROF_BEGIN
@@ -622,10 +623,18 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             }
             return true;
         });
+        // nothing of this warp's is in flight when tensor memory is freed, also where a wait ran out
+        if (elect_one()) {
+            if (PAIR) umma_commit_own_pair(smem_u32(&bars->retired));
+            else umma_commit(smem_u32(&bars->retired));
+        }
+        __syncwarp();
+        mbar_drain(smem_u32(&bars->retired), 0u);
         PROF_FLUSH(0)
     } else if (warp == 2) {
         // ── loader (TMA): activation tile, packed codes, scales ─────────────
         Ring r = {0, 0u};
+        int copied = 0, tiles = 0;                               // stages and tiles' scales this warp has started to copy
         PROF_DECL
         for_each_tile<SWIGLU, XR, SPLIT, PAIR>(a, p.nt_r, p.nt_x, [&](const TileInfo& t, int it) -> bool {
             const int ksteps = t.K / kTileK;
@@ -633,7 +642,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             tile_rows<SWIGLU>(a, t, t.ntile, mi0, mi1, row0, row1);
             const int sbuf = it & 1;
             PROF_BEGIN
-            if (!mbar_wait(smem_u32(&bars->sempty[sbuf]), (uint32_t)((it >> 1) & 1) ^ 1u, abort_flag)) return false;
+            if (!mbar_wait(smem_u32(&bars->sempty[sbuf]), (uint32_t)((it >> 1) & 1) ^ 1u, abort_flag, p.spin_limit)) return false;
             PROF_END(0)
             if (lane == 0) {
                 // bytes of one row of scales for this reduction length
@@ -655,13 +664,14 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                 }
             }
             __syncwarp();
+            ++tiles;
             // activation rows this tile needs: one box of 128 slots, a second one past 128 rows; of a pair, each
             // CTA brings its half of the slots
             const bool two = WIDE && !PAIR && t.rows > 128;
             const int xslot = t.slot0 + (PAIR ? (int)rank * (((t.rows + 31) & ~31) >> 1) : 0);
             for (int ks = 0; ks < ksteps; ++ks) {
                 PROF_BEGIN
-                if (!mbar_wait(smem_u32(&bars->empty[r.s]), r.ph ^ 1u, abort_flag)) return false;
+                if (!mbar_wait(smem_u32(&bars->empty[r.s]), r.ph ^ 1u, abort_flag, p.spin_limit)) return false;
                 PROF_END(1)
                 if (lane == 0) {
                     const uint32_t bar = smem_u32(&bars->qfull[r.s]);
@@ -680,9 +690,19 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                 }
                 __syncwarp();
                 r.advance(1, stages);
+                ++copied;
             }
             return true;
         });
+        // the copies still in flight where a wait ran out (else they were consumed long ago)
+        for (int i = min(copied, stages); i > 0; --i) {
+            if (--r.s < 0) {
+                r.s = stages - 1;
+                r.ph ^= 1u;
+            }
+            mbar_drain(smem_u32(&bars->qfull[r.s]), r.ph);
+        }
+        for (int it = max(0, tiles - 2); it < tiles; ++it) mbar_drain(smem_u32(&bars->sfull[it & 1]), (uint32_t)(it >> 1) & 1u);
         PROF_FLUSH(1)
     } else if ((warp >= 4 && warp < 8) || warp >= 16) {
         // ── epilogue ────────────────────────────────────────────────────────
@@ -739,7 +759,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
                 rf[0] = row_factor(t.extra ? S.x_down : S.down, S.dn_stride_s, t.ntile * 128 + lane128);
             }
             PROF_BEGIN
-            if (!mbar_wait(smem_u32(&bars->acc_full[buf]), (uint32_t)(round & 1), abort_flag)) return false;
+            if (!mbar_wait(smem_u32(&bars->acc_full[buf]), (uint32_t)(round & 1), abort_flag, p.spin_limit)) return false;
             PROF_END(0)
             tc_fence_after();
             PROF_BEGIN
@@ -993,7 +1013,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             const uint32_t s_addr = sc_base + (uint32_t)(sbuf * p.sc_bytes) + (uint32_t)qrow * srow;
             const uint32_t b_addr = s_addr + 128u * srow;
             PROF_BEGIN
-            if (!mbar_wait(smem_u32(&bars->sfull[sbuf]), (uint32_t)((it >> 1) & 1), abort_flag)) return false;
+            if (!mbar_wait(smem_u32(&bars->sfull[sbuf]), (uint32_t)((it >> 1) & 1), abort_flag, p.spin_limit)) return false;
             PROF_END(0)
             int r_exp = 0;
             if (FMT == FMT_MXFP8) {
@@ -1013,7 +1033,7 @@ __device__ __forceinline__ void prefill_tc_body(const GroupedArgs& a, const TcPa
             int ks = grp_id;
             for (; ks < ksteps; ks += 2) {
                 PROF_BEGIN
-                if (!mbar_wait(smem_u32(&bars->qfull[r.s]), r.ph, abort_flag)) return false;
+                if (!mbar_wait(smem_u32(&bars->qfull[r.s]), r.ph, abort_flag, p.spin_limit)) return false;
                 PROF_END(1)
                 PROF_BEGIN
                 const uint32_t stage = sbase + (uint32_t)(r.s * p.stage_bytes);

@@ -39,6 +39,7 @@ struct Bars {                                      // shared-memory control bloc
     uint64_t acc_empty[2];
     uint64_t sfull[2];                             // scales of a tile landed
     uint64_t sempty[2];                            // ... and were consumed by all producer warps
+    uint64_t retired;                              // the MMA warp's last commit
     uint32_t tmem_base;
     int abort;
 };
@@ -55,6 +56,7 @@ struct TcParams {
     int sc_bytes;                                  // one tile's scale buffer
     int panel_bytes;                               // resident activation panel (0: streamed per stage)
     int lg_group;                                  // log2 of the group size
+    int spin_limit;                                // bound of every wait
     int epi_bytes;                                 // wide tiles: the epilogue warps' transposing buffers
     unsigned long long ord_lut;                    // reduction index at position p of a block of 16, 4 bits each
 };

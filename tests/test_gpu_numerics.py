@@ -97,6 +97,31 @@ def test_expired_router_wait_is_reported_and_shows_in_the_result(cuda):
     assert torch.equal(again, good)
 
 
+@pytest.mark.parametrize("bits,intermediate", [(4, 512), (4, 192), (6, 512)])
+def test_expired_wait_of_the_tensor_core_products_is_reported(cuda, bits, intermediate):
+    """Pairs of CTAs, single CTAs and two-term weights with waits that give up at once: the kernels return, the status
+    word says so, and the next call on the same workspace is correct."""
+    cfg = MoEConfig("give-up", tokens=300, hidden=512, num_experts=4, top_k=2, intermediate=intermediate, bits=bits,
+                    shared_intermediate=0, group_size=64 if intermediate == 512 else 32, seed=95)
+    x, p = make_params(cfg)
+    moe = moe_to_device(p, cuda)
+    xd = t_bf16(x, cuda)
+    good = moe.forward_with_stream(xd).clone()
+    moe.check_status()
+    lib = _lib.lib()
+    try:
+        lib.imx_testing_prefill_give_up(1)
+        moe.forward_with_stream(xd)
+        with pytest.raises(_lib.IronMLXError) as e:
+            moe.check_status()
+        assert e.value.code == _lib.ERR_DEVICE and "status 3" in str(e.value)
+    finally:
+        lib.imx_testing_prefill_give_up(0)
+    again = moe.forward_with_stream(xd)
+    moe.check_status()
+    assert torch.equal(again, good)
+
+
 def test_expired_handoff_wait_is_reported_and_the_gpu_stays_usable(cuda):
     """A bounded wait that runs out (the partial-sum flags of the decode kernels withheld by a test hook, the spin
     limit cut to 200 iterations): the kernels return, the status word says so, and the next call on the same
