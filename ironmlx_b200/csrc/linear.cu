@@ -33,7 +33,8 @@ namespace {
 // 2048 -> 152064 57 -> 51 us.  Block m: the identity slot order, the work units of the single expert (balanced,
 // at most unit_rows slots each) and cleared scheduler words.
 // SCALED: any bf16 row fits fp16 once its largest magnitude is brought into [2^14, 2^15) by a power of two, which
-// the output gets back: row_scale = 2^-k.  Rows of zeros and rows with NaNs stay as they are.  A row with infinities would
+// the output gets back: row_scale = 2^-k (what is below 2^-28 of the largest loses bits, below 2^-39 all of them; beside
+// the largest, fp32 sums keep 2^-24).  Rows of zeros and rows with NaNs stay as they are.  A row with infinities would
 // meet weights split into two terms, inf * hi + inf * lo, which is NaN wherever the signs differ: its products, infinities
 // by the sign of the weights that meet one (NaN for a zero or opposite ones), are written here, and a NaN for its factor
 // tells the product's epilogue to leave them.

@@ -149,9 +149,9 @@ bool tc_aligned(const ExpertSet& s, bool second_only) {
     return !s.has_extra || (ok(s.x_down) && (second_only || (ok(s.x_gate) && ok(s.x_up))));
 }
 
-// variant: 3 = two-term weights (the only one for the formats two_term_supported() names); 0 = the shipped configuration (tensor-memory operand, 256-slot tiles in both products), 1 =
-// tensor-memory operand, 128-slot tiles and streamed activations everywhere, 2 = as 1 with the dequantized
-// tile in shared memory (1, 2: cross-checks).
+// variant: 0 = the shipped configuration (tensor-memory operand, 256-slot tiles in both products), 3 = the same with
+// two-term weights, 1 = tensor-memory operand, 128-slot tiles and streamed activations everywhere, 2 = as 1 with the
+// dequantized tile in shared memory (1, 2: cross-checks).
 int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid, int variant) {
     IMX_REQUIRE(variant == 3 ? two_term_supported(a.set, a.second_only != 0)
                 : (variant == 0 && a.out16 == nullptr && tc_rows32_supported(a.set)) || prefill_tc_supported(a.set, a.second_only != 0),
@@ -211,8 +211,8 @@ int launch_prefill_tc(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid
     TcMaps mgu, mdn;
     std::memset(&mgu, 0, sizeof(mgu));
     if (!a.second_only)
-    IMX_TRY(make_tensor_map_2d(xsrc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (size_t)a.n_slots, (size_t)s.n_in, (size_t)s.n_in * 2, kTileK,
-                               128, true, &mgu.x));
+        IMX_TRY(make_tensor_map_2d(xsrc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (size_t)a.n_slots, (size_t)s.n_in, (size_t)s.n_in * 2,
+                                   kTileK, 128, true, &mgu.x));
     IMX_TRY(make_tensor_map_2d(a.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (size_t)a.n_slots, (size_t)mid_max, (size_t)a.act_stride * 2,
                                kTileK, 128, true, &mdn.x));
     // routed experts: gate and up rows live in one stacked matrix [E*2I, H]; down in [E*H, I]

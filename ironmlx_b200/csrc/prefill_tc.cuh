@@ -1,49 +1,38 @@
-// Prefill-regime grouped expert products on the 5th-generation tensor cores,
-// every MLX weight format the block accepts at these sizes (affine 2/4/8-bit,
-// mxfp8, nvfp4):
+// Grouped expert products on the 5th-generation tensor cores, every weight format: affine 2/4/8-bit, mxfp8 and nvfp4 as one
+// fp16 value a weight, affine 2/3/4/5/6/8-bit as the sum of two (TwoTerm below):
 //
 //   first product   act[slot, :] = silu(x W_gate^T) * (x W_up^T)       (moe.rs:26-30)
 //   second product  out[slot, :] = row_scale[slot] * (act W_down^T)    (moe.rs:31, 155-161)
 //
-// each the grouped form of `quantized_matmul(transpose = true)`
-// (mlx/src/nn/linear.rs:51-63), with `tcgen05.mma` (kind::f16, fp16 x fp16 ->
-// fp32) and the accumulator in tensor memory.
+// each the grouped form of `quantized_matmul(transpose = true)` (mlx/src/nn/linear.rs:51-63), with `tcgen05.mma`
+// (kind::f16, fp16 x fp16 -> fp32) and the accumulator in tensor memory.
 //
-// The WEIGHTS are the A operand (M = 128 weight rows, one tensor-memory lane
-// each), the sorted slots of one expert are the N side (N = the unit's rows
-// rounded up to 16, at most 128), K in steps of 64.  The packed weights are
-// dequantized by producer warps straight into TENSOR MEMORY (`tcgen05.st`), and
-// the MMA takes A from there: the dequantized tile never passes through shared
-// memory, which the 128 x 128 tile of an smem-smem MMA saturates (the measured
-// limit of the kernel this one replaces).  Shared memory carries only what the
-// copy engine brings: the activation tile (B operand, 128-byte swizzle) and
-// the packed codes.  A variant with the dequantized tile in shared memory
-// (TS = false) is kept as a cross-check.
+// The WEIGHTS are the A operand (M = 128 weight rows, one tensor-memory lane each; 256 in a pair of CTAs), the sorted
+// slots of one expert are the N side (the unit's rows rounded up to 16 or 32, at most 256), K in steps of 64.  The packed
+// weights are dequantized by producer warps straight into TENSOR MEMORY (`tcgen05.st`), and the MMA takes A from there:
+// the dequantized tile never passes through shared memory, which the 128 x 128 tile of an smem-smem MMA saturates.  Shared
+// memory carries only what the copy engine brings: the activation tile (B operand, 128-byte swizzle) and the packed
+// codes.  A variant with the dequantized tile in shared memory (TS = false) is kept as a cross-check.
 //
-// One persistent CTA per SM, 16 warps, specialised:
-//   warp 0        issues the MMAs (one elected lane), commits a stage back to
-//                 the loader and the finished accumulator to the epilogue (two
-//                 accumulators: the epilogue of tile i overlaps the MMAs of i+1)
+// One persistent CTA per SM, 20 warps, specialised:
+//   warp 0        issues the MMAs (one elected lane; of a pair, CTA 0's), commits a stage back to the loader and the
+//                 finished accumulator to the epilogue
 //   warp 1        allocates / frees tensor memory
-//   warp 2        loader: tiled TMA copies of the activation tile, the packed
-//                 codes (two boxes of 64 rows) per K step and, once per tile,
-//                 the tile's scale (and bias) rows
-//   warps 4..7    epilogue: tcgen05.ld of their 32 lanes; lane = weight row,
-//                 column = slot.  First product: gate row j sits on lane
-//                 16 q + l, the matching up row on lane 16 q + l + 16 of the same
-//                 warp, so SwiGLU needs one shuffle exchange and no shared memory
-//   warps 8..15   producers, two groups of four warps on alternating K steps; a
-//                 thread owns one weight row: its 16/32/64 bytes of codes ->
-//                 64 fp16 values (exact codes, one HFMA2 / HMUL2 with the
-//                 group's scale) -> one tcgen05.st of 32 columns
-// Every wait is bounded; on expiry the CTA records a status, every role leaves
-// its loop and tensor memory is freed.  Wide tiles run in clusters of two CTAs (PAIR below); no multicast loads.
+//   warp 2        loader: tiled TMA copies of the activation tile and the packed codes (two boxes of 64 rows) per K step
+//                 and, once per tile, the tile's scale (and bias) rows as runs of bytes
+//   warps 4..7    epilogue, and 16..19 for the other half of a wide tile's slots (or the other accumulator): tcgen05.ld,
+//                 16-bit rows turned round in shared memory and stored 16 bytes at a time.  First product: in every 16
+//                 lanes eight hold gate rows and eight the matching up rows, so that a thread gets both values of a
+//                 (row, slot) and SwiGLU needs no exchange
+//   warps 8..15   producers, two groups of four warps on alternating K steps; a thread owns one weight row: its 16 to 64
+//                 bytes of codes -> 64 fp16 values (or pairs of them) -> tcgen05.st of 32 columns (two-term: 64)
+// Every wait is bounded; on expiry the CTA records a status, every role leaves its loop, what is in flight is waited for
+// and tensor memory is freed.  Wide tiles run in clusters of two CTAs (PAIR below); no multicast loads.
 //
-// Scales: affine rounds s*q+b once to fp16.  nvfp4: q * (e4m3 block scale) is
-// exact in fp16, the fp32 tensor scale is applied in the epilogue.  mxfp8: the
-// e4m3 value times 2^(s - r), r the largest scale exponent of the weight row,
-// is exact in fp16 (down to 2^-24 of the row's largest magnitude); 2^(r - 127)
-// is applied per row in the epilogue.
+// Scales: affine rounds s*q+b once to fp16 (two terms: to 22 bits).  nvfp4: q * (e4m3 block scale) is exact in fp16, the
+// fp32 tensor scale is applied in the epilogue.  mxfp8: the e4m3 value times 2^(s - r), r the largest scale exponent of
+// the weight row, is exact in fp16 (down to 2^-24 of the row's largest magnitude); 2^(r - 127) is applied per row in the
+// epilogue.
 #pragma once
 #include <cuda.h>
 
@@ -400,16 +389,22 @@ struct Dequant<FMT_NVFP4> {
 
 // ── two-term weights ────────────────────────────────────────────────────────
 // The formats no 16-bit kernel serves (affine 3/5/6-bit, groups of 32) had their weights in fp32 in the scalar kernel, and
-// the decode kernels keep affine weights exact.  One fp16 rounding of s * q + b would be a loss, so the MMA gets the weight as a sum of two
-// fp16 terms, hi + lo, good to 22 bits, with two MMAs per 16 values: the tile of A is 64 tensor-memory columns per
-// K step.  Everything is exact but the last rounding of lo:
-//   p = rn(q * s), e = q * s - p           exact: s is a bf16 value (8 bits), q has at most 6
-//   hi = rn(p + b), lo = rn(e + err)       err = the rounding error of p + b (two-sum)
+// the decode kernels keep affine weights exact.  One fp16 rounding of s * q + b would be a loss, so the MMA gets the weight
+// as a sum of two fp16 terms, hi + lo, good to 22 bits, with two MMAs per 16 values: the tile of A is 64 tensor-memory
+// columns per K step.  Everything is exact but the last rounding of lo:
+//   p = rn(q * s), e = q * s - p           exact: q and s have 8 bits at most, what p (11 bits) leaves of 16 fits e
+//   hi = rn(p + b), lo = rn(e + err)       err = the rounding error of p + b (Knuth's two-sum)
 // fp16's range is met by a power of two 2^k per weight row, from the row's largest |s| 2^bits or |b|, taken back in
-// the epilogue (fp32).  Measured on a B200 against the scalar kernels, 1000 tokens over 256 experts of 2048 x 512, 6-bit:
-// both products 5.65 ms -> 0.48 ms (the block 5.73 -> 0.54 ms); what bounds it now is the dequantization: twelve
-// half-precision operations a pair of values in eight warps, two thirds of a K step's time.  Codes are pulled out in pairs (a, a + D) of a window of the bit stream, so that the second
-// one lands in the upper half-word HS bits up (that factor goes into its copy of the scale); codes of a block of 16
+// the epilogue (fp32); scales below 2^-21 of that lose bits to fp16's subnormals, an absolute error of 2^-38 of the row's
+// largest weight.  Infinite or NaN scales make the whole row NaN.  Error against fp64, 2-norm, two terms / scalar kernel:
+// 2048 x 8192 6-bit, 100 rows 1.659308e-3 / 1.659305e-3 of the output, nearly all of it the rounding to bf16; fp32 rows
+// of the expert stage 2.068e-4 / 2.067e-4, the fp16 SwiGLU rows' (what is more comes from the tensor cores' sums, which
+// truncate: 7e-6).
+// Measured on a B200 against the scalar kernels, 1000 tokens over 256 experts of 2048 x 512, 6-bit: both products 5.65 ms ->
+// 0.48 ms (the block 5.73 -> 0.54 ms); what bounds it now is the dequantization: twelve half-precision operations a pair
+// of values in eight warps, two thirds of a K step's time.  From one row on: 1 token 206 -> 83 us a block, a row through
+// 2048 x 4096 86 -> 34 us.  Codes are pulled out in pairs (a, a + D) of a window of the bit stream, so that the second one
+// lands in the upper half-word HS bits up (that factor goes into its copy of the scale); codes of a block of 16
 // that have no partner at that distance pair with their neighbour.
 template <int BITS>
 struct TwoTerm {
@@ -1160,15 +1155,15 @@ int configure() {
         IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
         return IMX_OK;
     } else {
-    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    return IMX_OK;
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<true, FMT, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc_kernel<false, FMT, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        return IMX_OK;
     }
 }
 
@@ -1183,7 +1178,8 @@ int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, co
     if (a.out_bf16 != nullptr) {
         if (dn.pair) prefill_pair_kernel<false, FMT, true><<<sms & ~1, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
         else if (dn.wide) prefill_tc_kernel<false, FMT, true, true, false, true><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
-        else if constexpr (!two_term(FMT)) prefill_tc_kernel<false, FMT, true, false, false, true><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        else if constexpr (!two_term(FMT))
+            prefill_tc_kernel<false, FMT, true, false, false, true><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
         IMX_LAUNCHED();
         IMX_CHECK_CUDA(cudaGetLastError());
         return IMX_OK;
@@ -1202,23 +1198,23 @@ int launch_fmt(const GroupedArgs& a, const Plan& gu, const Plan& dn, bool ts, co
         IMX_CHECK_CUDA(cudaGetLastError());
         return IMX_OK;
     } else {
-    if (!a.second_only) {
-        if (gu.pair) prefill_pair_kernel<true, FMT><<<sms & ~1, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
-        else if (!ts) prefill_tc_kernel<true, FMT, false, false, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
-        else if (gu.wide) prefill_tc_kernel<true, FMT, true, true, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
-        else prefill_tc_kernel<true, FMT, true, false, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+        if (!a.second_only) {
+            if (gu.pair) prefill_pair_kernel<true, FMT><<<sms & ~1, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+            else if (!ts) prefill_tc_kernel<true, FMT, false, false, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+            else if (gu.wide) prefill_tc_kernel<true, FMT, true, true, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+            else prefill_tc_kernel<true, FMT, true, false, false><<<sms, kThreadsTc, gu.smem, stream>>>(a, gu.p, mgu);
+            IMX_LAUNCHED();
+            IMX_CHECK_CUDA(cudaGetLastError());
+        }
+        if (mid) IMX_CHECK_CUDA(cudaEventRecord(mid, stream));
+        if (dn.pair) prefill_pair_kernel<false, FMT><<<sms & ~1, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        else if (!ts) prefill_tc_kernel<false, FMT, false, false, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        else if (dn.wide) prefill_tc_kernel<false, FMT, true, true, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        else if (dn.xr) prefill_tc_kernel<false, FMT, true, false, true><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
+        else prefill_tc_kernel<false, FMT, true, false, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
         IMX_LAUNCHED();
         IMX_CHECK_CUDA(cudaGetLastError());
-    }
-    if (mid) IMX_CHECK_CUDA(cudaEventRecord(mid, stream));
-    if (dn.pair) prefill_pair_kernel<false, FMT><<<sms & ~1, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
-    else if (!ts) prefill_tc_kernel<false, FMT, false, false, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
-    else if (dn.wide) prefill_tc_kernel<false, FMT, true, true, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
-    else if (dn.xr) prefill_tc_kernel<false, FMT, true, false, true><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
-    else prefill_tc_kernel<false, FMT, true, false, false><<<sms, kThreadsTc, dn.smem, stream>>>(a, dn.p, mdn);
-    IMX_LAUNCHED();
-    IMX_CHECK_CUDA(cudaGetLastError());
-    return IMX_OK;
+        return IMX_OK;
     }
 }
 

@@ -16,15 +16,18 @@ constexpr uint32_t kTmemCols = 512;                // two 128-column accumulator
 constexpr uint32_t kTmemA = 256;                   // first column of the A ring (32 columns per stage)
 constexpr int kThreadsTc = 640;                    // 20 warps: 4 control, 4 + 4 epilogue, 8 producers
 
-// FMT_T*: affine weights as a two-term fp16 sum (hi + lo), see TwoTerm below.
-enum { FMT_A4 = 0, FMT_A8 = 1, FMT_A2 = 2, FMT_MXFP8 = 3, FMT_NVFP4 = 4, FMT_T2 = 5, FMT_T3 = 6, FMT_T4 = 7, FMT_T5 = 8, FMT_T6 = 9, FMT_T8 = 10 };
+// FMT_T*: affine weights as a two-term fp16 sum (hi + lo), see TwoTerm in prefill_tc.cuh.
+enum { FMT_A4 = 0, FMT_A8 = 1, FMT_A2 = 2, FMT_MXFP8 = 3, FMT_NVFP4 = 4,
+       FMT_T2 = 5, FMT_T3 = 6, FMT_T4 = 7, FMT_T5 = 8, FMT_T6 = 9, FMT_T8 = 10 };
 __host__ __device__ constexpr bool two_term(int fmt) { return fmt >= FMT_T2; }
 __host__ __device__ constexpr int two_term_bits(int fmt) { return fmt == FMT_T8 ? 8 : fmt - FMT_T2 + 2; }
 // Bytes of one row the copy engine brings per K step of 64 values.  3- and 5-bit rows advance by 24 and 40 bytes a
 // step and a copy starts on a multiple of 16: the box starts at the multiple below and is wide enough for both
 // positions.  48-byte rows spread eight lanes' 16-byte loads over all banks without a swizzle.
 __host__ __device__ constexpr int q_row_bytes(int fmt) {
-    return fmt == FMT_A8 || fmt == FMT_MXFP8 || fmt == FMT_T8 ? 64 : (fmt == FMT_A2 || fmt == FMT_T2 ? 16 : (fmt == FMT_T3 || fmt == FMT_T5 || fmt == FMT_T6 ? 48 : 32));
+    if (fmt == FMT_A8 || fmt == FMT_MXFP8 || fmt == FMT_T8) return 64;
+    if (fmt == FMT_A2 || fmt == FMT_T2) return 16;
+    return fmt == FMT_T3 || fmt == FMT_T5 || fmt == FMT_T6 ? 48 : 32;
 }
 // First byte of K step ks's box in a packed row (a multiple of 16).
 __host__ __device__ constexpr int q_step_byte(int fmt, int ks) {
