@@ -208,7 +208,9 @@ __device__ __forceinline__ int permuted_pos(int i) {
     return (int)((lut >> (4 * i)) & 0xf);
 }
 
-template <int BITS, bool SWIGLU>
+// BF16: the rows leave rounded to bf16 (the second product alone), in kernels of their own: with the choice made at run time
+// the blocks' decode kernels lost up to 1 %.
+template <int BITS, bool SWIGLU, bool BF16>
 __device__ __forceinline__ void epilogue(const GroupedArgs& a, const TaskCtx& c, float (&acc)[2][4], int g, int t) {
     if (c.valid) {
         if (SWIGLU) {
@@ -235,7 +237,7 @@ __device__ __forceinline__ void epilogue(const GroupedArgs& a, const TaskCtx& c,
                         const int slot = c.slot0 + slot_l;
                         const float sc = a.row_scale ? a.row_scale[slot] : 1.f;
                         const float v = acc[T][i] * c.gs[T] * sc;
-                        if (a.out_bf16 != nullptr) a.out_bf16[(size_t)slot * a.set.n_in + row] = __float2bfloat16_rn(v);
+                        if (BF16) a.out_bf16[(size_t)slot * a.set.n_in + row] = __float2bfloat16_rn(v);
                         else a.out[(size_t)slot * a.set.n_in + row] = v;
                     }
                 }

@@ -255,7 +255,7 @@ __device__ __forceinline__ void compute(const FpStage<MX>& st, const FpTask& c, 
     }
 }
 
-template <bool SWIGLU>
+template <bool SWIGLU, bool BF16>
 __device__ __forceinline__ void finish(const GroupedArgs& a, const FpTask& c, float (&acc)[2][2][4], int g, int t) {
     if (c.n_it > 0) {
         float r[2][4];
@@ -281,7 +281,7 @@ __device__ __forceinline__ void finish(const GroupedArgs& a, const FpTask& c, fl
                     if (slot_l < c.rows) {
                         const int slot = c.slot0 + slot_l;
                         const float sc = a.row_scale ? a.row_scale[slot] : 1.f;
-                        if (a.out_bf16 != nullptr) a.out_bf16[(size_t)slot * a.set.n_in + row] = __float2bfloat16_rn(r[T][i] * sc);
+                        if (BF16) a.out_bf16[(size_t)slot * a.set.n_in + row] = __float2bfloat16_rn(r[T][i] * sc);
                         else a.out[(size_t)slot * a.set.n_in + row] = r[T][i] * sc;
                     }
                 }
@@ -295,7 +295,9 @@ __device__ __forceinline__ void finish(const GroupedArgs& a, const FpTask& c, fl
             for (int i = 0; i < 4; ++i) acc[T][h][i] = 0.f;
 }
 
-template <bool MX, bool SWIGLU>
+// BF16: rows rounded to bf16 (the second product alone), a kernel of its own as in decode_common.cuh: 81 tokens over 256
+// experts in mxfp8 248.6 -> 245.5 us a block as a graph.
+template <bool MX, bool SWIGLU, bool BF16 = false>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 decode_fp_kernel(const GroupedArgs a, const int pairs_per_unit) {
     const int lane = threadIdx.x & 31;
@@ -328,7 +330,7 @@ decode_fp_kernel(const GroupedArgs a, const int pairs_per_unit) {
             for (int i = 0; i < 4; ++i) acc[T][h][i] = 0.f;
     auto advance_compute = [&]() {
         while (c_task < task_hi && c_it >= cc.n_it) {
-            finish<SWIGLU>(a, cc, acc, g, t);
+            finish<SWIGLU, BF16>(a, cc, acc, g, t);
             ++c_task;
             c_it = 0;
             if (c_task < task_hi) setup_task<MX, SWIGLU>(a, c_task, pairs_per_unit, g, t, cc);
@@ -375,7 +377,8 @@ int launch_mode(const GroupedArgs& a, cudaStream_t stream, cudaEvent_t mid) {
         IMX_CHECK_CUDA(cudaGetLastError());
     }
     if (mid) IMX_CHECK_CUDA(cudaEventRecord(mid, stream));
-    decode_fp_kernel<MX, false><<<sms * kCtasPerSm, kThreads, 0, stream>>>(a, s.n_in / 32); IMX_LAUNCHED();
+    auto second = a.out_bf16 != nullptr ? decode_fp_kernel<MX, false, true> : decode_fp_kernel<MX, false>;
+    second<<<sms * kCtasPerSm, kThreads, 0, stream>>>(a, s.n_in / 32); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     return IMX_OK;
 }

@@ -125,7 +125,7 @@ __device__ __forceinline__ void compute(const Stage<BITS>& st, const TaskCtx& c,
     }
 }
 
-template <int BITS, bool SWIGLU>
+template <int BITS, bool SWIGLU, bool BF16 = false>
 __global__ void __launch_bounds__(kThreads, 1)
 decode_mma_kernel(const GroupedArgs a, const int pairs_per_unit, const int g128) {
     const int lane = threadIdx.x & 31;
@@ -157,7 +157,7 @@ decode_mma_kernel(const GroupedArgs a, const int pairs_per_unit, const int g128)
         for (int i = 0; i < 4; ++i) acc[T][i] = 0.f;
     auto advance_compute = [&]() {
         while (c_task < task_hi && c_it >= cc.n_it) {
-            epilogue<BITS, SWIGLU>(a, cc, acc, g, t);
+            epilogue<BITS, SWIGLU, BF16>(a, cc, acc, g, t);
             ++c_task;
             c_it = 0;
             if (c_task < task_hi) setup_task<BITS, SWIGLU>(a, c_task, pairs_per_unit, g, t, g128, cc);
@@ -205,7 +205,8 @@ int launch_bits(const GroupedArgs& a, int g128, cudaStream_t stream, cudaEvent_t
         IMX_CHECK_CUDA(cudaGetLastError());
     }
     if (mid) IMX_CHECK_CUDA(cudaEventRecord(mid, stream));
-    decode_mma_kernel<BITS, false><<<grid, kThreads, 0, stream>>>(a, s.n_in / 32, g128); IMX_LAUNCHED();
+    auto second = a.out_bf16 != nullptr ? decode_mma_kernel<BITS, false, true> : decode_mma_kernel<BITS, false>;
+    second<<<grid, kThreads, 0, stream>>>(a, s.n_in / 32, g128); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     return IMX_OK;
 }

@@ -580,7 +580,8 @@ struct Chunk {
     int slot;                // parts > 1: the pair's hand-off slot
 };
 
-template <int kWarps, int kStages>
+// BF16: rows rounded to bf16 (the second product alone), a kernel of its own as in decode_common.cuh.
+template <int kWarps, int kStages, bool BF16>
 __global__ void __launch_bounds__(kWarps * 32, 1)
 decode_second_kernel(const GroupedArgs a, const DecodeParams p, const __grid_constant__ DecodeMaps maps) {
     constexpr int kSmemW = kWarps * kStages * kWBytes, kSmemS = kWarps * kStages * kSBytes;
@@ -821,11 +822,10 @@ decode_second_kernel(const GroupedArgs a, const DecodeParams p, const __grid_con
                     const int slot_l = 2 * t + sl;
                     const int row = c_pair * 32 + T * 16 + 2 * g;
                     const float sc = kUnscale * (sl ? c_rs1 : c_rs0);
-                    if (slot_l >= c_unit.rows) continue;
-                    if (a.out_bf16 != nullptr)
+                    if (BF16 && slot_l < c_unit.rows)
                         *reinterpret_cast<__nv_bfloat162*>(a.out_bf16 + (size_t)(c_unit.slot0 + slot_l) * S.n_in + row) =
                             __floats2bfloat162_rn(acc[T][sl] * sc, acc[T][2 + sl] * sc);
-                    else
+                    if (!BF16 && slot_l < c_unit.rows)
                         *reinterpret_cast<float2*>(a.out + (size_t)(c_unit.slot0 + slot_l) * S.n_in + row) =
                             make_float2(acc[T][sl] * sc, acc[T][2 + sl] * sc);
                 }
@@ -1015,7 +1015,8 @@ int launch_with(const GroupedArgs& a, const DecodeMaps& gu, const DecodeMaps& dn
     if (device_needs_setup(di.ordinal, kSetupDecodeTmap)) {      // once per device, outside any stream capture
         constexpr int most = (int)smem_bytes(kWarps, kStages, kMaxSumGroups);
         IMX_CHECK_CUDA(cudaFuncSetAttribute(decode_first_kernel<kWarps, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-        IMX_CHECK_CUDA(cudaFuncSetAttribute(decode_second_kernel<kWarps, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(decode_second_kernel<kWarps, kStages, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        IMX_CHECK_CUDA(cudaFuncSetAttribute(decode_second_kernel<kWarps, kStages, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
         device_mark_setup(di.ordinal, kSetupDecodeTmap);
     }
     const int grid = sms;
@@ -1064,7 +1065,8 @@ int launch_with(const GroupedArgs& a, const DecodeMaps& gu, const DecodeMaps& dn
     }
     if (mid) IMX_CHECK_CUDA(cudaEventRecord(mid, stream));
     // second product: the group sums of a unit's SwiGLU rows come from the sums of 16 the first product left
-    decode_second_kernel<kWarps, kStages><<<grid, kWarps * 32, smem_dn, stream>>>(a, pd, dn); IMX_LAUNCHED();
+    auto second = a.out_bf16 != nullptr ? decode_second_kernel<kWarps, kStages, true> : decode_second_kernel<kWarps, kStages, false>;
+    second<<<grid, kWarps * 32, smem_dn, stream>>>(a, pd, dn); IMX_LAUNCHED();
     IMX_CHECK_CUDA(cudaGetLastError());
     return IMX_OK;
 }
