@@ -189,9 +189,11 @@ bool decode_supported(const ExpertSet& s) { return decode_mma_supported(s) || de
 //     8-bit 8 rows 400 / 509, 16 rows 662 / 513; 2-bit 16 rows 538 / 464
 //   64 of 1024 x 512 and 128 of 1024 x 256 (3.5 an SM): mxfp8 8 rows 92 / 88; nvfp4 16 rows 79 / 87, 20 rows 90 / 88; 8-bit
 //     16 rows 106 / 126, 20 rows 132 / 126; 2-bit 16 rows 106 / 108, 20 rows 122 / 107; 4-bit 20 rows 113 / 117, 24 rows 124 / 121
-//   8 of 2048 x 1024 (0.9 an SM): mxfp8 8 rows 72 / 55; nvfp4 16 rows 52 / 54, 24 rows 57 / 55
-//   16 of 512 x 256 (0.4 an SM): mxfp8 31 rows 40 / 42, 64 rows 44 / 46, 100 rows 62 / 53; nvfp4 31 rows 33 / 41, 128 rows
-//     51 / 49; 8-bit 128 rows 62 / 59; one expert of 2048 x 512: mxfp8 8 rows 49 / 35, nvfp4 31 rows 31 / 35
+//   32 of 2048 x 512 (1.7 an SM): nvfp4 16 rows 88 / 84 (long reductions gain sooner than those of 1024)
+//   8 of 2048 x 1024 (0.9 an SM): mxfp8 8 rows 72 / 55; nvfp4 16 rows 45 / 45 (as a graph)
+//   16 of 512 x 256 (0.4 an SM): mxfp8 31 rows 40 / 42, 64 rows 44 / 46, 74 rows 62 / 51; as a graph, without the host's share
+//     of a launch more, 31 rows 33 / 33, 64 rows 43 / 41, 74 rows 53 / 41; nvfp4 31 rows 33 / 41, 128 rows 51 / 49; 8-bit 128
+//     rows 62 / 59; one expert of 2048 x 512: mxfp8 8 rows 49 / 35, nvfp4 31 rows 31 / 35
 //   affine 4-bit in groups of 64, tensor-map decode kernel: not below prefill sizes (28 rows 486 / 546)
 static bool tiles_per_sm(const ExpertSet& s, double at_least) {
     DeviceInfo di;
@@ -200,8 +202,8 @@ static bool tiles_per_sm(const ExpertSet& s, double at_least) {
 }
 static long rows32_from(const ExpertSet& s) {
     const bool few = !tiles_per_sm(s, 0.5);
-    if (s.fmt.mode == IMX_MODE_MXFP8) return (few && s.num_experts > 1 ? 96L : 8L) * s.num_experts;
-    return (few ? 128L : (tiles_per_sm(s, 8) ? 16L : 20L)) * s.num_experts;
+    if (s.fmt.mode == IMX_MODE_MXFP8) return (few && s.num_experts > 1 ? 65L : 8L) * s.num_experts;
+    return (few ? 128L : (tiles_per_sm(s, 8) || s.n_in >= 2048 ? 16L : 20L)) * s.num_experts;
 }
 static long two_term_from(const ExpertSet& s) {
     if (decode_tmap_supported(s)) return 1L << 40;
