@@ -267,10 +267,12 @@ route_splitk_kernel(const __nv_bfloat16* __restrict__ x, int n_tokens, int H, co
 // Second half of the split-K router: one warp per token adds the K slices in slice
 // order (so the sums do not depend on timing) and does softmax / top-k.
 // SORT: the CTA that gets here last sorts the assignments of all of them, every CTA clears its share of the scheduler
-// words.  For the smallest batches, where a launch of its own costs more than it sorts (a call of 1 token 52.5 -> 51.0 us,
-// of 19 tokens 95.1 -> 93.1); at 64 tokens the sixteen tokens a CTA of 512 threads finishes take longer than the launch
-// saved (119.4 -> 120.1 us as a graph), so that more than kRouteSortTokens keep four tokens a CTA and the sort's launch.
-constexpr int kFinThreadsSort = 512;
+// words.  For the smallest batches, where a launch of its own costs the host more than it sorts: a call of 1 token 52.5 ->
+// 50.5 us, of 19 tokens 95.1 -> 92 through Python.  As a graph the two are even, provided the tokens are spread over CTAs: nine
+// warps (one more than the scan over 256 experts needs) take 16 tokens of 256 experts 4-bit in 70.5 us where sixteen take
+// 72.0 and the sort's own launch 70.3.  At 64 tokens the sort's own launch is the faster one (119.4 / 120.1 with sixteen
+// warps), so that more than kRouteSortTokens keep four tokens a CTA.
+constexpr int kFinThreadsSort = 288;
 constexpr int kRouteSortTokens = 32;
 
 template <bool SORT>

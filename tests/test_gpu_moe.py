@@ -147,7 +147,7 @@ def test_reruns_are_bit_identical(cuda):
 
 
 @pytest.mark.parametrize("word", [1, 7, -1])
-@pytest.mark.parametrize("tokens", [5, 19])
+@pytest.mark.parametrize("tokens", [5, 9, 19, 32])
 def test_small_batches_do_not_rely_on_words_an_earlier_call_left(cuda, tokens, word):
     """The last CTA of the decode-size router sorts; it is found by a count in the workspace's status block, whatever
     value that word held before the call."""
